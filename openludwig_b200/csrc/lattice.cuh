@@ -32,6 +32,42 @@ __host__ __device__ inline float w_of(int k) {
                  : d2 == 1 ? 2.0f / 27.0f : d2 == 2 ? 1.0f / 54.0f : 1.0f / 216.0f;
 }
 
+// Reciprocal, quotient and square root of positive normal floats without a
+// slow path: the hardware approximation (PTX rcp / rsqrt.approx, documented
+// within about one unit in the last place), then one Newton-Raphson step on
+// an FMA residual (Markstein, IBM J. Res. Dev. 34, 1990), which leaves the
+// result within a hair of half a unit.  The operators `/` and sqrtf compile to
+// a range check and a call for the rare operands, and each such call ends a
+// basic block of the cell update; these stay in its straight line.
+__device__ __forceinline__ float recip_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float recip_nr(float x) {
+  const float r = recip_approx(x);
+  return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
+__device__ __forceinline__ float quotient_nr(float a, float b) {
+  const float r = recip_approx(b);
+  const float q = a * r;
+  return fmaf(fmaf(-b, q, a), r, q);
+}
+__device__ __forceinline__ float sqrt_nr(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  const float s = x * y;
+  return fmaf(fmaf(-s, s, x), 0.5f * y, s);
+}
+// x / 3, correctly rounded for normal results: the product with the rounded
+// third, corrected by the exact remainder (Markstein's theorem for constant
+// divisors).
+__device__ __forceinline__ float third_of(float x) {
+  const float c = 0.333333343f;  // the float nearest 1/3
+  const float q = x * c;
+  return fmaf(fmaf(-3.0f, q, x), c, q);
+}
+
 // O(u^2) equilibrium, physics_utils.jl:19-24.
 __device__ __forceinline__ float feq2(float rho, float ux, float uy, float uz,
                                       float w, float cx, float cy, float cz) {

@@ -316,7 +316,7 @@ __device__ __forceinline__ float wale_from(const WaleVel &V, float c_wale) {
   const float gsq31 = g31 * g11 + g32 * g21 + g33 * g31;
   const float gsq32 = g31 * g12 + g32 * g22 + g33 * g32;
   const float gsq33 = g31 * g13 + g32 * g23 + g33 * g33;
-  const float tr_term = (gsq11 + gsq22 + gsq33) / 3.0f;
+  const float tr_term = third_of(gsq11 + gsq22 + gsq33);
   const float Sd11 = gsq11 - tr_term, Sd22 = gsq22 - tr_term, Sd33 = gsq33 - tr_term;
   const float Sd12 = 0.5f * (gsq12 + gsq21), Sd13 = 0.5f * (gsq13 + gsq31),
               Sd23 = 0.5f * (gsq23 + gsq32);
@@ -325,13 +325,14 @@ __device__ __forceinline__ float wale_from(const WaleVel &V, float c_wale) {
                     2.0f * (Sd12 * Sd12 + Sd13 * Sd13 + Sd23 * Sd23);
   const float OP2 = g11 * g11 + g22 * g22 + g33 * g33 +
                     2.0f * (S12 * S12 + S13 * S13 + S23 * S23);
-  float nu = 0.0f;
-  if (OP1 > 1e-12f) {
-    const float op1_32 = OP1 * sqrtf(OP1);
-    const float op2_52 = OP2 * OP2 * sqrtf(fmaxf(OP2, 1e-12f));
-    const float den = op2_52 + OP1 * sqrtf(sqrtf(fmaxf(OP1, 1e-12f)));
-    if (den > 1e-12f) nu = (c_wale * c_wale) * op1_32 / den;
-  }
+  // evaluated unconditionally (the floor keeps the roots defined) and selected:
+  // a branch here would split the cell update's instruction schedule
+  const float o1 = fmaxf(OP1, 1e-12f);
+  const float r1 = sqrt_nr(o1);
+  const float op2_52 = OP2 * OP2 * sqrt_nr(fmaxf(OP2, 1e-12f));
+  const float den = op2_52 + o1 * sqrt_nr(r1);
+  const float nu = (OP1 > 1e-12f && den > 1e-12f)
+                       ? quotient_nr((c_wale * c_wale) * (o1 * r1), den) : 0.0f;
   return nu;
 }
 
@@ -378,22 +379,61 @@ __device__ __forceinline__ void wall_force(float dist, float rho, float ux, floa
 // ---------------------------------------------------------------------------
 // Chimera transforms (kernel_cumulant.jl:4-26) and the cumulant collision
 // (kernel_cumulant.jl:330-559).  A holds populations on entry and on exit.
+//
+// The cell update is bound by instruction issue and by the latency of its
+// dependent chains, not by memory, so it is written for few instructions and
+// straight-line code:
+//   * the raw x-moments are formed first, in place; rho and the momentum are
+//     sums over them (26 additions instead of 78) and the first transform
+//     continues from them;
+//   * a triple's zeroth moment reuses its second (m0 = b + m2);
+//   * reciprocals, quotients and roots are the branch-free forms below
+//     instead of calls with a slow path, so the scheduler sees one block;
+//   * with omega_3 = omega_4 = 1 (the reference's defaults) every third-order
+//     moment and every C_211 kind is relaxed to exactly zero, so its forward
+//     transform, the fifth-order products and the zero terms of the backward
+//     transform are left out (collide_cumulant<true>).
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void raw_moments(float &a, float &b, float &c) {
+  const float m2 = a + c, m1 = c - a;
+  a = b + m2;
+  b = m1;
+  c = m2;
+}
+// Raw moments (m0, m1, m2) of a triple -> central ones about u.
+__device__ __forceinline__ void centre(float m0, float &b, float &c, float u) {
+  const float m1 = b;
+  b = fmaf(-u, m0, m1);
+  c = fmaf(u * u, m0, fmaf(-2.0f * u, m1, c));
+}
 __device__ __forceinline__ void chim_fwd(float &a, float &b, float &c, float u) {
-  const float m0 = a + b + c, m1 = c - a, m2 = a + c;
-  a = m0;
-  b = m1 - u * m0;
-  c = m2 - 2.0f * u * m1 + u * u * m0;
+  raw_moments(a, b, c);
+  centre(a, b, c, u);
 }
 // (m2 +- m1) / 2 as fma(+-1/2, m1, m2 / 2): the same bits (halving is exact
 // at these magnitudes, so both round the same exact value once), one
 // instruction fewer.
 __device__ __forceinline__ void chim_bwd(float &a, float &b, float &c, float u) {
-  const float m0 = a, m1 = b + u * a, m2 = c + 2.0f * u * b + u * u * a;
+  const float m0 = a, m1 = fmaf(u, a, b), m2 = fmaf(u * u, a, fmaf(2.0f * u, b, c));
   const float h = 0.5f * m2;
   c = fmaf(0.5f, m1, h);
   a = fmaf(-0.5f, m1, h);
   b = m0 - m2;
+}
+// The same for a zero first moment ...
+__device__ __forceinline__ void chim_bwd_b0(float &a, float &b, float &c, float u) {
+  const float m0 = a, m1 = u * a, m2 = fmaf(u * u, a, c);
+  const float h = 0.5f * m2;
+  c = fmaf(0.5f, m1, h);
+  a = fmaf(-0.5f, m1, h);
+  b = m0 - m2;
+}
+// ... and for a triple that holds a first moment only.
+__device__ __forceinline__ void chim_bwd_b(float &a, float &b, float &c, float u) {
+  const float m1 = b, h = u * b;
+  c = fmaf(0.5f, m1, h);
+  a = fmaf(-0.5f, m1, h);
+  b = -2.0f * h;
 }
 
 struct CumulantRates {
@@ -401,11 +441,14 @@ struct CumulantRates {
   int limiter;
 };
 
-__device__ __forceinline__ void collide_cumulant(float A[27], float ux, float uy,
-                                                 float uz, const CumulantRates &r) {
+// A holds raw x-moments on entry (raw_moments over the consecutive triples)
+// and populations on exit.  LOW: omega3 == omega4 == 1.
+template <bool LOW>
+__device__ __forceinline__ void collide_cumulant(float (&A)[27], float ux, float uy, float uz,
+                                                 const CumulantRates &r) {
   // forward: x (consecutive triples), then y (stride 3), then z (stride 9)
 #pragma unroll
-  for (int i = 0; i < 9; ++i) chim_fwd(A[3 * i], A[3 * i + 1], A[3 * i + 2], ux);
+  for (int i = 0; i < 9; ++i) centre(A[3 * i], A[3 * i + 1], A[3 * i + 2], ux);
 #pragma unroll
   for (int zz = 0; zz < 3; ++zz)
 #pragma unroll
@@ -415,22 +458,15 @@ __device__ __forceinline__ void collide_cumulant(float A[27], float ux, float uy
   for (int i = 0; i < 9; ++i) chim_fwd(A[i], A[i + 9], A[i + 18], uz);
 
   const float k000 = A[0];
-  const float inv_r = 1.0f / fmaxf(k000, 0.01f);
+  const float inv_r = recip_nr(fmaxf(k000, 0.01f));
   // index of central moment (a,b,c) = a + 3b + 9c
   const float c200 = A[2] * inv_r, c020 = A[6] * inv_r, c002 = A[18] * inv_r;
   const float c110 = A[4] * inv_r, c101 = A[10] * inv_r, c011 = A[12] * inv_r;
-  const float c210 = A[5] * inv_r, c120 = A[7] * inv_r, c201 = A[11] * inv_r;
-  const float c021 = A[15] * inv_r, c102 = A[19] * inv_r, c012 = A[21] * inv_r;
-  const float c111 = A[13] * inv_r;
   const float c220n = A[8] * inv_r, c202n = A[20] * inv_r, c022n = A[24] * inv_r;
-  const float c211n = A[14] * inv_r, c121n = A[16] * inv_r, c112n = A[22] * inv_r;
 
   const float C220 = c220n - c200 * c020 - 2.0f * c110 * c110;
   const float C202 = c202n - c200 * c002 - 2.0f * c101 * c101;
   const float C022 = c022n - c020 * c002 - 2.0f * c011 * c011;
-  const float C211 = c211n - c200 * c011 - 2.0f * c110 * c101;
-  const float C121 = c121n - c020 * c101 - 2.0f * c110 * c011;
-  const float C112 = c112n - c002 * c110 - 2.0f * c101 * c011;
 
   const float cs2 = 0.333333333f;
   const float om1 = r.omega1, omb = r.omega_bulk;
@@ -438,63 +474,104 @@ __device__ __forceinline__ void collide_cumulant(float A[27], float ux, float uy
   const float Dtr_s = (1.0f - omb) * Dtr + omb * (3.0f * cs2);
   const float D1s = (1.0f - om1) * (c200 - c020);
   const float D2s = (1.0f - om1) * (c200 - c002);
-  const float c200s = (Dtr_s + D1s + D2s) / 3.0f;
-  const float c020s = (Dtr_s - 2.0f * D1s + D2s) / 3.0f;
-  const float c002s = (Dtr_s + D1s - 2.0f * D2s) / 3.0f;
+  const float c200s = third_of(Dtr_s + D1s + D2s);
+  const float c020s = third_of(Dtr_s - 2.0f * D1s + D2s);
+  const float c002s = third_of(Dtr_s + D1s - 2.0f * D2s);
   float c110s = (1.0f - om1) * c110;
   float c101s = (1.0f - om1) * c101;
   float c011s = (1.0f - om1) * c011;
   if (r.limiter == OL_LIMITER_FACTORED) {
-    const float b110 = sqrtf(fmaxf(c200s * c020s, 0.0f));
-    const float b101 = sqrtf(fmaxf(c200s * c002s, 0.0f));
-    const float b011 = sqrtf(fmaxf(c020s * c002s, 0.0f));
+    // (a floor far below any product's rounding keeps the root defined)
+    const float b110 = sqrt_nr(fmaxf(c200s * c020s, 1e-36f));
+    const float b101 = sqrt_nr(fmaxf(c200s * c002s, 1e-36f));
+    const float b011 = sqrt_nr(fmaxf(c020s * c002s, 1e-36f));
     c110s = fminf(fmaxf(c110s, -b110), b110);
     c101s = fminf(fmaxf(c101s, -b101), b101);
     c011s = fminf(fmaxf(c011s, -b011), b011);
   }
-  const float o3 = 1.0f - r.omega3;
-  const float c210s = o3 * c210, c120s = o3 * c120, c201s = o3 * c201;
-  const float c021s = o3 * c021, c102s = o3 * c102, c012s = o3 * c012;
-  const float c111s = o3 * c111;
-  const float o4d = 1.0f - r.omega4_diag, o4 = 1.0f - r.omega4;
+  const float o4d = 1.0f - r.omega4_diag;
   const float C220s = o4d * C220, C202s = o4d * C202, C022s = o4d * C022;
-  const float C211s = o4 * C211, C121s = o4 * C121, C112s = o4 * C112;
-
-  const float c220s = C220s + c200s * c020s + 2.0f * c110s * c110s;
-  const float c202s = C202s + c200s * c002s + 2.0f * c101s * c101s;
-  const float c022s = C022s + c020s * c002s + 2.0f * c011s * c011s;
-  const float c211s = C211s + c200s * c011s + 2.0f * c110s * c101s;
-  const float c121s = C121s + c020s * c101s + 2.0f * c110s * c011s;
-  const float c112s = C112s + c002s * c110s + 2.0f * c101s * c011s;
-  const float c221s = c200s * c021s + c020s * c201s + 4.0f * c110s * c111s +
-                      2.0f * c101s * c120s + 2.0f * c011s * c210s;
-  const float c212s = c200s * c012s + c002s * c210s + 2.0f * c110s * c102s +
-                      4.0f * c101s * c111s + 2.0f * c011s * c201s;
-  const float c122s = c020s * c102s + c002s * c120s + 2.0f * c110s * c012s +
-                      4.0f * c011s * c111s + 2.0f * c101s * c021s;
-  float c222s = c200s * C022s + c020s * C202s + c002s * C220s +
-                4.0f * (c110s * C112s + c101s * C121s + c011s * C211s);
-  c222s += 2.0f * (c210s * c012s + c201s * c021s + c120s * c102s) + 4.0f * c111s * c111s;
-  c222s += c200s * c020s * c002s +
-           2.0f * (c200s * c011s * c011s + c020s * c101s * c101s + c002s * c110s * c110s) +
-           8.0f * c110s * c101s * c011s;
-
   const float rr = k000;
-  A[0] = rr;
-  A[1] = 0.0f; A[3] = 0.0f; A[9] = 0.0f;
-  A[2] = rr * c200s; A[6] = rr * c020s; A[18] = rr * c002s;
-  A[4] = rr * c110s; A[10] = rr * c101s; A[12] = rr * c011s;
-  A[5] = rr * c210s; A[7] = rr * c120s; A[11] = rr * c201s;
-  A[15] = rr * c021s; A[19] = rr * c102s; A[21] = rr * c012s;
-  A[13] = rr * c111s;
-  A[8] = rr * c220s; A[20] = rr * c202s; A[24] = rr * c022s;
-  A[14] = rr * c211s; A[16] = rr * c121s; A[22] = rr * c112s;
-  A[17] = rr * c221s; A[23] = rr * c212s; A[25] = rr * c122s;
-  A[26] = rr * c222s;
+  if constexpr (LOW) {
+    // e = C + 2 c^2 of each pair; t = 2 c110 c101 is shared by 211 and 222
+    const float e220 = fmaf(2.0f * c110s, c110s, C220s);
+    const float e202 = fmaf(2.0f * c101s, c101s, C202s);
+    const float e022 = fmaf(2.0f * c011s, c011s, C022s);
+    const float c220s = fmaf(c200s, c020s, e220);
+    const float c202s = fmaf(c200s, c002s, e202);
+    const float c022s = fmaf(c020s, c002s, e022);
+    const float t = 2.0f * c110s * c101s;
+    const float c211s = fmaf(c200s, c011s, t);
+    const float c121s = fmaf(c020s, c101s, 2.0f * c110s * c011s);
+    const float c112s = fmaf(c002s, c110s, 2.0f * c101s * c011s);
+    const float c222s =
+        fmaf(c002s, c220s, fmaf(c200s, e022, fmaf(c020s, e202, 4.0f * t * c011s)));
+    A[0] = rr;
+    A[2] = rr * c200s; A[6] = rr * c020s; A[18] = rr * c002s;
+    A[4] = rr * c110s; A[10] = rr * c101s; A[12] = rr * c011s;
+    A[8] = rr * c220s; A[20] = rr * c202s; A[24] = rr * c022s;
+    A[14] = rr * c211s; A[16] = rr * c121s; A[22] = rr * c112s;
+    A[26] = rr * c222s;
+    // backward z: (a, b) lines; odd total order is zero
+    chim_bwd_b0(A[0], A[9], A[18], uz);
+    chim_bwd_b0(A[2], A[11], A[20], uz);
+    chim_bwd_b0(A[4], A[13], A[22], uz);
+    chim_bwd_b0(A[6], A[15], A[24], uz);
+    chim_bwd_b0(A[8], A[17], A[26], uz);
+    chim_bwd_b(A[1], A[10], A[19], uz);
+    chim_bwd_b(A[3], A[12], A[21], uz);
+    chim_bwd_b(A[5], A[14], A[23], uz);
+    chim_bwd_b(A[7], A[16], A[25], uz);
+  } else {
+    const float c210 = A[5] * inv_r, c120 = A[7] * inv_r, c201 = A[11] * inv_r;
+    const float c021 = A[15] * inv_r, c102 = A[19] * inv_r, c012 = A[21] * inv_r;
+    const float c111 = A[13] * inv_r;
+    const float c211n = A[14] * inv_r, c121n = A[16] * inv_r, c112n = A[22] * inv_r;
+    const float C211 = c211n - c200 * c011 - 2.0f * c110 * c101;
+    const float C121 = c121n - c020 * c101 - 2.0f * c110 * c011;
+    const float C112 = c112n - c002 * c110 - 2.0f * c101 * c011;
+    const float o3 = 1.0f - r.omega3;
+    const float c210s = o3 * c210, c120s = o3 * c120, c201s = o3 * c201;
+    const float c021s = o3 * c021, c102s = o3 * c102, c012s = o3 * c012;
+    const float c111s = o3 * c111;
+    const float o4 = 1.0f - r.omega4;
+    const float C211s = o4 * C211, C121s = o4 * C121, C112s = o4 * C112;
 
-  // backward: z, then y, then x
+    const float c220s = C220s + c200s * c020s + 2.0f * c110s * c110s;
+    const float c202s = C202s + c200s * c002s + 2.0f * c101s * c101s;
+    const float c022s = C022s + c020s * c002s + 2.0f * c011s * c011s;
+    const float c211s = C211s + c200s * c011s + 2.0f * c110s * c101s;
+    const float c121s = C121s + c020s * c101s + 2.0f * c110s * c011s;
+    const float c112s = C112s + c002s * c110s + 2.0f * c101s * c011s;
+    const float c221s = c200s * c021s + c020s * c201s + 4.0f * c110s * c111s +
+                        2.0f * c101s * c120s + 2.0f * c011s * c210s;
+    const float c212s = c200s * c012s + c002s * c210s + 2.0f * c110s * c102s +
+                        4.0f * c101s * c111s + 2.0f * c011s * c201s;
+    const float c122s = c020s * c102s + c002s * c120s + 2.0f * c110s * c012s +
+                        4.0f * c011s * c111s + 2.0f * c101s * c021s;
+    float c222s = c200s * C022s + c020s * C202s + c002s * C220s +
+                  4.0f * (c110s * C112s + c101s * C121s + c011s * C211s);
+    c222s += 2.0f * (c210s * c012s + c201s * c021s + c120s * c102s) + 4.0f * c111s * c111s;
+    c222s += c200s * c020s * c002s +
+             2.0f * (c200s * c011s * c011s + c020s * c101s * c101s + c002s * c110s * c110s) +
+             8.0f * c110s * c101s * c011s;
+
+    A[0] = rr;
+    A[1] = 0.0f; A[3] = 0.0f; A[9] = 0.0f;
+    A[2] = rr * c200s; A[6] = rr * c020s; A[18] = rr * c002s;
+    A[4] = rr * c110s; A[10] = rr * c101s; A[12] = rr * c011s;
+    A[5] = rr * c210s; A[7] = rr * c120s; A[11] = rr * c201s;
+    A[15] = rr * c021s; A[19] = rr * c102s; A[21] = rr * c012s;
+    A[13] = rr * c111s;
+    A[8] = rr * c220s; A[20] = rr * c202s; A[24] = rr * c022s;
+    A[14] = rr * c211s; A[16] = rr * c121s; A[22] = rr * c112s;
+    A[17] = rr * c221s; A[23] = rr * c212s; A[25] = rr * c122s;
+    A[26] = rr * c222s;
+    // backward z
 #pragma unroll
-  for (int i = 0; i < 9; ++i) chim_bwd(A[i], A[i + 9], A[i + 18], uz);
+    for (int i = 0; i < 9; ++i) chim_bwd(A[i], A[i + 9], A[i + 18], uz);
+  }
+  // backward y, then x
 #pragma unroll
   for (int zz = 0; zz < 3; ++zz)
 #pragma unroll
@@ -1107,6 +1184,12 @@ __device__ __forceinline__ void stream_collide_cell(const LevelDev &L, const int
   collide_cell<OP, ST, WALE>(L, nbbase, A, b, t, obs, spg);
 }
 
+// Device watchdog of the native path: non-finite or vanishing density.
+__device__ __forceinline__ void watchdog(int32_t *status, float rho) {
+  if (!(fabsf(rho) < 1e30f)) atomicOr(status, 1);
+  else if (rho < 0.01f) atomicOr(status, 2);
+}
+
 // Everything after the pull: bounce-back, moments, sponge, wall model,
 // WALE, collision, forcing and the stores of cell t of block b.
 template <int OP, class ST, bool WALE>
@@ -1118,27 +1201,41 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
   const size_t own = (size_t)nbbase[13] + t;
   const GlobalOut<ST> out(L, own);
 
-  float rho = 0.0f, jx = 0.0f, jy = 0.0f, jz = 0.0f;
-#pragma unroll
-  for (int k = 0; k < 27; ++k) {
-    rho += A[k];
-    if (cx_of(k) == 1) jx += A[k]; else if (cx_of(k) == -1) jx -= A[k];
-    if (cy_of(k) == 1) jy += A[k]; else if (cy_of(k) == -1) jy -= A[k];
-    if (cz_of(k) == 1) jz += A[k]; else if (cz_of(k) == -1) jz -= A[k];
-  }
-  // Note: jx += v*cx in the reference equals jx +/- v exactly for cx = +/-1.
-  if (L.status) {  // device watchdog (native path): report, never trap
-    if (!(fabsf(rho) < 1e30f)) atomicOr(L.status, 1);
-    else if (rho < 0.01f) atomicOr(L.status, 2);
-  }
-
+  float rho, jx, jy, jz;
   if (obs) {
+    if (L.status) {
+      rho = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 27; ++k) rho += A[k];
+      watchdog(L.status, rho);
+    }
     out.macro(1.0f, 0.0f, 0.0f, 0.0f);
     out.template f_all<true>(A);
     return;
   }
-  rho = fmaxf(rho, 0.01f);
-  const float inv_rho = 1.0f / rho;
+  if constexpr (OP == OL_OP_CUMULANT) {
+    // A becomes the raw x-moments (m0, m1, m2) of each (y, z) triple
+#pragma unroll
+    for (int i = 0; i < 9; ++i) raw_moments(A[3 * i], A[3 * i + 1], A[3 * i + 2]);
+    const float s0 = A[0] + A[3] + A[6], s1 = A[9] + A[12] + A[15], s2 = A[18] + A[21] + A[24];
+    rho = s0 + s1 + s2;
+    jx = (A[1] + A[4] + A[7]) + (A[10] + A[13] + A[16]) + (A[19] + A[22] + A[25]);
+    jy = (A[6] - A[0]) + (A[15] - A[9]) + (A[24] - A[18]);
+    jz = s2 - s0;
+  } else {
+    rho = jx = jy = jz = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 27; ++k) {
+      rho += A[k];
+      if (cx_of(k) == 1) jx += A[k]; else if (cx_of(k) == -1) jx -= A[k];
+      if (cy_of(k) == 1) jy += A[k]; else if (cy_of(k) == -1) jy -= A[k];
+      if (cz_of(k) == 1) jz += A[k]; else if (cz_of(k) == -1) jz -= A[k];
+    }
+  }
+  // device watchdog (native path): report, never trap
+  if (L.status) watchdog(L.status, rho);
+  rho = fminf(fmaxf(rho, 0.01f), 3e38f);
+  const float inv_rho = recip_nr(rho);
   float ux = jx * inv_rho, uy = jy * inv_rho, uz = jz * inv_rho;
   if (spg > 0.0f) {
     rho = rho * (1.0f - spg) + 1.0f * spg;
@@ -1147,10 +1244,15 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
     uz = uz * (1.0f - spg);
     if (sp.sponge_blend_distributions == 1) {
 #pragma unroll
-      for (int k = 0; k < 27; ++k) {
-        const float ft = feq_auto(1.0f, sp.u_inlet, 0.0f, 0.0f, w_of(k), (float)cx_of(k),
-                                  (float)cy_of(k), (float)cz_of(k), sp.compressible_corr);
-        A[k] = A[k] * (1.0f - spg) + ft * spg;
+      for (int i = 0; i < 9; ++i) {
+        float ft[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          ft[j] = feq_auto(1.0f, sp.u_inlet, 0.0f, 0.0f, w_of(3 * i + j), (float)cx_of(3 * i + j),
+                           (float)cy_of(3 * i + j), (float)cz_of(3 * i + j), sp.compressible_corr);
+        if (OP == OL_OP_CUMULANT) raw_moments(ft[0], ft[1], ft[2]);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) A[3 * i + j] = A[3 * i + j] * (1.0f - spg) + ft[j] * spg;
       }
     }
   }
@@ -1171,9 +1273,9 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
 
   float omega;  // omega_1 (cumulant) or omega (BGK)
   if (OP == OL_OP_CUMULANT) {
-    const float nu_mol = (sp.tau_molecular - 0.5f) / 3.0f;
+    const float nu_mol = third_of(sp.tau_molecular - 0.5f);
     const float tau_eff = 0.5f + 3.0f * (nu_mol + nu_eddy);
-    omega = 1.0f / fmaxf(tau_eff, 0.500001f);
+    omega = recip_nr(fminf(fmaxf(tau_eff, 0.500001f), 3e38f));
     CumulantRates r;
     r.omega1 = omega;
     r.omega_bulk = sp.omega_bulk;
@@ -1182,11 +1284,12 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
     r.omega4_diag = sp.omega_4;
     if (sp.adaptive_omega4 == 1) {
       const float om1m2 = omega - 2.0f;
-      const float Av = -(om1m2 * om1m2) / (sp.lambda_param * omega + 1e-10f);
+      const float Av = quotient_nr(-(om1m2 * om1m2), sp.lambda_param * omega + 1e-10f);
       r.omega4_diag = fminf(fmaxf(Av, 0.01f), 2.0f);
     }
     r.limiter = sp.limiter_type;
-    collide_cumulant(A, uxe, uye, uze, r);
+    if (sp.omega_3 == 1.0f && sp.omega_4 == 1.0f) collide_cumulant<true>(A, uxe, uye, uze, r);
+    else collide_cumulant<false>(A, uxe, uye, uze, r);
     if (sp.limiter_type == OL_LIMITER_POSITIVITY) {
       float fmin = A[0];
 #pragma unroll
@@ -1198,7 +1301,7 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
     // c.u_eq, as kernel_cumulant.jl:610 does (the reference line 302 names
     // an undefined `cu`).
     const float tau_turb = sp.tau_molecular + nu_eddy * 3.0f;
-    omega = 1.0f / fmaxf(tau_turb, 0.500001f);
+    omega = recip_nr(fminf(fmaxf(tau_turb, 0.500001f), 3e38f));
     float Pxx = 0.f, Pyy = 0.f, Pzz = 0.f, Pxy = 0.f, Pyz = 0.f, Pzx = 0.f;
 #pragma unroll
     for (int k = 0; k < 27; ++k) {
