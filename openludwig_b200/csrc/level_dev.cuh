@@ -67,6 +67,7 @@ struct LevelDev {
   ol_step_params sp;
   int32_t *status;        // device watchdog word (may be null)
   const uint32_t *halo_tab;  // staging table (stream_collide.cuh)
+  const uint32_t *ghost_units;  // unit table of the ghost pass (stream_collide.cuh)
   float *ghost;           // absent-neighbour pull sources, kHaloEntries per row, or null
   const int32_t *gidx;    // block -> ghost row (-1: none); null = row b for block b
   // Pairing of the two child sub-steps of one parent step (kGhost* below):
@@ -94,6 +95,8 @@ struct WorkItem {
 // Per-device staging table of the 3176 out-of-block pull sources of a block
 // (built once on first use; see stage_block).
 const uint32_t *halo_table_device();
+// Per-device unit table of the ghost pass (null on failure).
+const uint32_t *ghost_units_device();
 // Per-device fault word of the warp-specialised kernels (null on failure).
 int *fault_word_device();
 // Current ol_set_stream_collide_kernel choice (OL_SC_KERNEL_*).

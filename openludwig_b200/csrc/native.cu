@@ -678,8 +678,8 @@ static int rebuild(ol_ctx *c) {
   std::vector<int32_t> bcount;         // links of each Bouzidi list
   int64_t scratch_max = 0;
   const int64_t dstride = c->capacity * BCELLS;
-  const uint32_t *tab = halo_table_device();
-  if (!tab) return set_error(OL_ERR_CUDA, "staging table allocation failed");
+  const uint32_t *tab = halo_table_device(), *gtab = ghost_units_device();
+  if (!tab || !gtab) return set_error(OL_ERR_CUDA, "staging table allocation failed");
   int64_t per_step = 2;  // advance + tick
 
   for (const auto &sl : slots) {
@@ -713,6 +713,7 @@ static int rebuild(ol_ctx *c) {
       L.sp.store_post_collision = 0;
       L.status = &c->d_cases[cs.slot].status;
       L.halo_tab = tab;
+      L.ghost_units = gtab;
       if (l > 1) {
         const DevLevel &PV = cs.levels[l - 2];
         L.sp.tau_parent = PV.tau;
@@ -746,6 +747,7 @@ static int rebuild(ol_ctx *c) {
         D.tp.nx_global = cs.nx * sc; D.tp.ny_global = cs.ny * sc; D.tp.nz_global = cs.nz * sc;
         D.tp.store_post_collision = 0;
         D.halo_tab = tab;
+        D.ghost_units = gtab;
         if (l > 1) {
           const DevLevel &PV = cs.levels[l - 2];
           D.tp.tau_g_parent = PV.tau_g;

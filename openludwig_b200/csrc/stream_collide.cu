@@ -43,15 +43,68 @@ static std::vector<uint32_t> build_halo_table() {
   return tab;
 }
 
-const uint32_t *halo_table_device() {
-  static std::mutex mu;
-  static uint32_t *per_dev[64] = {};
+// Unit table of the ghost pass (stream_collide.cuh).
+static std::vector<uint32_t> build_ghost_units() {
+  const std::vector<uint32_t> halo = build_halo_table();
+  std::vector<int> slot_of(27 * EPL, -1);  // [k][10^3 slot] -> staging-table entry
+  for (int i = 0; i < kHaloEntries; ++i)
+    slot_of[(halo[i] & 31) * EPL + (halo[i] >> 19)] = i;
+  std::vector<uint32_t> units, groups;
+  for (int order = 1; order <= 3; ++order)  // faces, edges, corners
+    for (int dir = 0; dir < 27; ++dir) {
+      const int o[3] = {cx_of(dir), cy_of(dir), cz_of(dir)};
+      if (o[0] * o[0] + o[1] * o[1] + o[2] * o[2] != order) continue;
+      int lo[3], hi[3];  // pair indices of the direction's groups per axis
+      for (int a = 0; a < 3; ++a) {
+        lo[a] = o[a] < 0 ? 0 : (o[a] > 0 ? 5 : 1);
+        hi[a] = o[a] < 0 ? 0 : (o[a] > 0 ? 5 : 4);
+      }
+      const uint32_t q0 = (uint32_t)groups.size();
+      for (int pz = lo[2]; pz <= hi[2]; ++pz)
+        for (int py = lo[1]; py <= hi[1]; ++py)
+          for (int px = lo[0]; px <= hi[0]; ++px)
+            groups.push_back((uint32_t)(px + 6 * py + 36 * pz) | (uint32_t)dir << 8);
+      for (int k = 0; k < 27; ++k) {
+        // pulled across the face, edge or corner: c_a = -o_a where o_a != 0
+        const int c[3] = {cx_of(k), cy_of(k), cz_of(k)};
+        bool pulls = true;
+        for (int a = 0; a < 3; ++a) pulls = pulls && (o[a] == 0 || c[a] == -o[a]);
+        if (!pulls) continue;
+        for (uint32_t q = q0; q < groups.size(); ++q) {
+          const uint32_t code = groups[q] & 255;
+          const int p[3] = {(int)code % 6, (int)(code / 6) % 6, (int)code / 36};
+          uint32_t slot[4];
+          for (int sub = 0; sub < 4; ++sub) {
+            int bits = sub, s[3];
+            for (int a = 0; a < 3; ++a) {
+              if (p[a] == 0) s[a] = -1;
+              else if (p[a] == 5) s[a] = 8;
+              else { s[a] = 2 * p[a] - 2 + (bits & 1); bits >>= 1; }
+            }
+            const int i = bits ? -1 : slot_of[k * EPL + e_index(s[0], s[1], s[2])];
+            slot[sub] = i < 0 ? (uint32_t)kGhostNoSlot : (uint32_t)i;
+          }
+          units.push_back((uint32_t)k | q << 5 | code << 13 | (uint32_t)dir << 21);
+          units.push_back(slot[0] | slot[1] << 16);
+          units.push_back(slot[2] | slot[3] << 16);
+          units.push_back(0);
+        }
+      }
+    }
+  units.insert(units.end(), groups.begin(), groups.end());
+  return units;
+}
+
+// A host table copied to the current device once and kept there (null on failure).
+template <int N>
+static const uint32_t *table_on_device(uint32_t *(&per_dev)[64], std::mutex &mu,
+                                       std::vector<uint32_t> (*build)()) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
   std::lock_guard<std::mutex> lk(mu);
   if (!per_dev[dev]) {
-    const std::vector<uint32_t> tab = build_halo_table();
-    if ((int)tab.size() != kHaloTableSize) return nullptr;
+    const std::vector<uint32_t> tab = build();
+    if ((int)tab.size() != N) return nullptr;
     uint32_t *d = nullptr;
     if (cudaMalloc(&d, tab.size() * sizeof(uint32_t)) != cudaSuccess) return nullptr;
     if (cudaMemcpy(d, tab.data(), tab.size() * sizeof(uint32_t), cudaMemcpyHostToDevice) !=
@@ -62,6 +115,17 @@ const uint32_t *halo_table_device() {
     per_dev[dev] = d;
   }
   return per_dev[dev];
+}
+
+const uint32_t *halo_table_device() {
+  static std::mutex mu;
+  static uint32_t *per_dev[64] = {};
+  return table_on_device<kHaloTableSize>(per_dev, mu, build_halo_table);
+}
+const uint32_t *ghost_units_device() {
+  static std::mutex mu;
+  static uint32_t *per_dev[64] = {};
+  return table_on_device<kGhostTableWords>(per_dev, mu, build_ghost_units);
 }
 
 // Loader table of the warp-specialised kernel (ws.cuh): the staging table's
@@ -101,22 +165,7 @@ static std::vector<uint32_t> build_ws_table() {
 const uint32_t *ws_table_device() {
   static std::mutex mu;
   static uint32_t *per_dev[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lk(mu);
-  if (!per_dev[dev]) {
-    const std::vector<uint32_t> tab = build_ws_table();
-    if ((int)tab.size() != kWsTableTotal) return nullptr;
-    uint32_t *d = nullptr;
-    if (cudaMalloc(&d, tab.size() * sizeof(uint32_t)) != cudaSuccess) return nullptr;
-    if (cudaMemcpy(d, tab.data(), tab.size() * sizeof(uint32_t), cudaMemcpyHostToDevice) !=
-        cudaSuccess) {
-      cudaFree(d);
-      return nullptr;
-    }
-    per_dev[dev] = d;
-  }
-  return per_dev[dev];
+  return table_on_device<kWsTableTotal>(per_dev, mu, build_ws_table);
 }
 
 // Per-device fault word of the warp-specialised kernels (bits kWsFault*):
@@ -388,7 +437,8 @@ extern "C" int ol_stream_collide(const ol_level_view *lv, const ol_parent_view *
   OL_CHECK_ARG((int64_t)lv->n_blocks * BCELLS < (1LL << 31),
                "ol_stream_collide: n_blocks too large for 32-bit plane offsets");
   L.halo_tab = halo_table_device();
-  if (!L.halo_tab) return set_error(OL_ERR_CUDA, "ol_stream_collide: staging table allocation failed");
+  L.ghost_units = ghost_units_device();
+  if (!L.halo_tab || !L.ghost_units) return set_error(OL_ERR_CUDA, "ol_stream_collide: staging table allocation failed");
   if (!sp->is_level_1) {
     OL_CHECK_ARG(pv && pv->f && pv->rho && pv->vel && pv->block_ptr && pv->n_blocks > 0,
                  "ol_stream_collide: fine level needs a parent view");

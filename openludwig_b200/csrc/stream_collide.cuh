@@ -178,39 +178,6 @@ __device__ __forceinline__ float interp_population(const LevelDev &L, int k,
   return finish_population(L, k, v, P.wx, P.wy, P.wz, r);
 }
 
-// The same population for both child sub-steps of a parent step from one
-// read of the parent's old and new state: g0 at weight 0 (the old state),
-// g1 at kSecondSubstepWeight; r0 / r1 are the moments at those weights.
-// Bitwise what interp_population gives at each weight.
-template <class ST>
-__device__ __forceinline__ void interp_population_pair(const LevelDev &L, int k,
-                                                       const ParentStencil &P,
-                                                       const float (&r0)[4],
-                                                       const float (&r1)[4], float &g0,
-                                                       float &g1) {
-  const bool temporal = L.sp.use_temporal_interp == 1;
-  using T = typename ST::T;
-  const T *po = (const T *)L.pf_old + (size_t)k * L.p_dstride;   // plane k
-  const T *pn = (const T *)L.pf + (size_t)k * L.p_dstride;
-  float v0[8], v1[8];
-#pragma unroll
-  for (int s = 0; s < 8; ++s) {
-    v0[s] = v1[s] = w_of(k);
-    if (P.ci[s] >= 0) {
-      const uint32_t c = (uint32_t)P.ci[s];
-      const float fn = ST::load(pn, c, k, L.p_inv_scale);
-      const float fo = temporal ? ST::load(po, c, k, L.p_inv_scale) : fn;
-      v0[s] = fo;
-      v1[s] = temporal ? lerp_rn(fo, fn, kSecondSubstepWeight) : fn;
-    }
-  }
-#pragma unroll
-  for (int s = 1; s < 8; ++s)
-    if (P.ci[s] < 0) { v0[s] = v0[0]; v1[s] = v1[0]; }
-  g0 = finish_population(L, k, v0, P.wx, P.wy, P.wz, r0);
-  g1 = finish_population(L, k, v1, P.wx, P.wy, P.wz, r1);
-}
-
 // ---------------------------------------------------------------------------
 // Source value of a pull whose neighbour block is absent and whose source
 // lies outside the domain or on level 1 (kernel_cumulant.jl:117-159); the
@@ -726,16 +693,42 @@ __device__ __noinline__ void fill_missing_flow(const LevelDev &L, const int *nbb
 
 // Separate pass over the blocks of a level: the absent-neighbour pull sources
 // of block b, in staging-table order, into L.ghost[b * kHaloEntries + i].
-// Same values as fill_missing_flow; here the CTA is small, leaves the SM's
-// L1 to the parent gathers (a parent cell serves ~20 ghost slots), keeps the
-// whole parent stencil of each ring position in shared memory, and spreads
-// only the slots that need a value over its threads (compacted lists), so no
-// stream-collide CTA waits at a barrier while a few of its threads
-// interpolate.  Parent cell indices are kept as int32 (the launch checks
-// that the parent's cells fit).
+// Same values as fill_missing_flow, from fewer gathers.  Fine cells 2m+1 and
+// 2m+2 of an axis interpolate between the same parent cells m and m+1, so the
+// 488 ring positions of a block fall into 152 groups (up to 2 x 2 positions)
+// that share their 8 parent cells.  The unit of work is one direction of one
+// group -- 1016 units for the 3176 slots -- and reads the 8 parent values
+// once for its up to 4 slots (and both sub-steps of a pair).  A fine block
+// touches at most 2 parent blocks per axis, so its 8 parent block ids are read
+// once, next to the neighbour row, and a stencil costs no table lookups.
+// The pass waits on gathers: per block there are three dependent round trips
+// (neighbour row, moments, populations) instead of a stencil chain per
+// position, and a third of the population gathers.  Measured per coarse step:
+// cube_3lvl (3 passes) 193 -> 119 us, the two passes of sphere_ddf 58 + 58 ->
+// 36 + 35 us; 256 threads at 4 CTAs per SM beat 3 CTAs with 80 registers (134)
+// and 128 threads at 6 CTAs (139) in spite of a few spilled words.
 constexpr int kGhostThreads = 256;
 constexpr int kGhostMinBlocks = 4;  // resident CTAs per SM (64 registers per thread)
-constexpr int kGhostScan = (kHaloEntries + kGhostThreads - 1) / kGhostThreads;  // 13
+constexpr int kGhostGroups = 152, kGhostUnits = 1016;
+constexpr int kGhostScan = (kGhostUnits + kGhostThreads - 1) / kGhostThreads;  // 4
+// Unit table: per unit one uint4 {k | group << 5 | code << 13 | direction << 21,
+// slots of positions 0 and 1, slots of positions 2 and 3 (16 bits each, 0xFFFF:
+// none), 0}, sorted by direction (faces, edges, corners), then per group one
+// word code | direction << 8.
+constexpr int kGhostNoSlot = 0xFFFF;
+constexpr int kGhostTableWords = 4 * kGhostUnits + kGhostGroups;
+// Group code: pair indices p (0..5 per axis, x fastest) of positions -1 |
+// 0,1 | 2,3 | 4,5 | 6,7 | 8.  Position `sub` of a group: its bits pick the
+// member on the axes that have two, x first.  Returns the position's
+// coordinate and trilinear weight along one axis and consumes a bit of sub.
+__device__ __forceinline__ int ghost_member(int p, int &sub, float &w) {
+  if (p == 0) { w = 0.75f; return -1; }
+  if (p == 5) { w = 0.25f; return 8; }
+  const int bit = sub & 1;
+  sub >>= 1;
+  w = bit ? 0.75f : 0.25f;
+  return 2 * p - 2 + bit;
+}
 
 // Warp-aggregated append of `value` to a shared list when `flag` is set;
 // every lane of the warp makes the call.
@@ -769,9 +762,17 @@ __device__ __forceinline__ float *ghost_next_row_of(const DEV &L, int b) {
 // What the ghost pass needs to know of a flow level; the thermal DDF
 // provides the same functions for its populations (thermal.cuh).
 __device__ __forceinline__ const ol_step_params &ghost_params(const LevelDev &L) { return L.sp; }
-__device__ __forceinline__ void ghost_corner_moments(const LevelDev &L, uint32_t c, float tw,
-                                                     float (&m)[4]) {
-  corner_moments(L, c, tw, m);
+// Parent planes of moment m (0: rho, 1..3: u) and of population k, new and old.
+__device__ __forceinline__ const float *ghost_moment_plane(const LevelDev &L, int m, bool old) {
+  if (m == 0) return old ? L.prho_old : L.prho;
+  return (old ? L.pvel_old : L.pvel) + (size_t)(m - 1) * L.p_dstride;
+}
+__device__ __forceinline__ const void *ghost_parent(const LevelDev &L, bool old) {
+  return old ? L.pf_old : L.pf;
+}
+__device__ __forceinline__ float ghost_finish(const LevelDev &L, int k, const float (&v)[8],
+                                              float wx, float wy, float wz, const float (&r)[4]) {
+  return finish_population(L, k, v, wx, wy, wz, r);
 }
 __device__ __forceinline__ void ghost_moments(const LevelDev &L, const ParentStencil &P, float tw,
                                               float (&r)[4]) {
@@ -783,16 +784,20 @@ __device__ __forceinline__ float ghost_population(const LevelDev &L, int k, cons
   return interp_population<ST>(L, k, P, r, tw);
 }
 template <class ST>
-__device__ __forceinline__ void ghost_population_pair(const LevelDev &L, int k,
-                                                      const ParentStencil &P,
-                                                      const float (&r0)[4], const float (&r1)[4],
-                                                      ST, float &g0, float &g1) {
-  interp_population_pair<ST>(L, k, P, r0, r1, g0, g1);
-}
-template <class ST>
 __device__ __forceinline__ float ghost_boundary(const LevelDev &L, int k, int b, int x, int y,
                                                 int z, ST) {
   return pull_boundary<ST>(L, k, b, x, y, z);
+}
+
+// A slot of a block that lies partly outside the domain (sizes that are no
+// multiple of 8) but is itself inside it: interpolated on its own.
+template <class ST, class DEV>
+__device__ __noinline__ float ghost_slot(const DEV &L, int k, int gx, int gy, int gz, float tw) {
+  ParentStencil P;
+  parent_stencil(L, gx, gy, gz, P);
+  float r[4];
+  ghost_moments(L, P, tw, r);
+  return ghost_population(L, k, P, r, tw, ST{});
 }
 
 // One CTA of kGhostThreads threads evaluates block b's row G.  With
@@ -802,121 +807,165 @@ __device__ __forceinline__ float ghost_boundary(const LevelDev &L, int k, int b,
 // of G are already set and only the domain-boundary slots are evaluated.
 template <class ST, class DEV>
 __device__ __forceinline__ void ghost_fill_block(const DEV &L, int b, float *G, float *G2) {
-  __shared__ int nbbase[27];
-  __shared__ int n_pos, n_slot;
-  __shared__ float rs[4][kRingEntries];     // interpolated rho, ux, uy, uz
-  __shared__ float rs2[4][kRingEntries];    // the same at the second sub-step's weight
-  __shared__ int32_t cs[8][kRingEntries];   // parent stencil cells
-  __shared__ float ws[3][kRingEntries];     // trilinear weights
-  __shared__ uint8_t iface_of[kRingEntries];  // ring position takes coarse-to-fine values
-  __shared__ int16_t pos_list[kRingEntries];
-  __shared__ int16_t slot_list[kHaloEntries];
+  using T = typename ST::T;
+  __shared__ int8_t kind[27];      // by direction: 0 nothing to do, 1 interpolate, 2 per slot
+  __shared__ int32_t pbase[8];     // first cell of the 2 x 2 x 2 parent blocks, -1 absent
+  __shared__ int n_unit;
+  __shared__ int16_t unit_list[kGhostUnits];
+  __shared__ float rs[4][4 * kGhostGroups];   // rho, ux, uy, uz per group position
+  __shared__ float rs2[4][4 * kGhostGroups];  // the same at the second sub-step's weight
   const int t = threadIdx.x;
   const auto &sp = ghost_params(L);
   const bool precomputed = L.ghost_mode == kGhostPairSecond;
-  const int mx = L.map_x[b], my = L.map_y[b], mz = L.map_z[b];
-  int missing = 0;
-  if (t < 27) {
-    const int nb = L.nbr[b + L.nbr_stride * t];
-    nbbase[t] = nb > 0 ? (int)((L.block_offset + nb - 1) * BCELLS) : -1;
-    missing = nb <= 0;
-    if (missing && precomputed) {
-      // the second sub-step of a pair only revisits absent neighbours that are
-      // not wholly inside the domain (all others are coarse-to-fine, set)
-      const int nbx = mx + t % 3 - 1, nby = my + (t / 3) % 3 - 1, nbz = mz + t / 9 - 1;
-      missing = !(nbx >= 1 && nbx * BS <= sp.nx_global && nby >= 1 &&
-                  nby * BS <= sp.ny_global && nbz >= 1 && nbz * BS <= sp.nz_global);
-    }
-  }
-  if (t == 0) { n_pos = 0; n_slot = 0; }
-  if (!__syncthreads_or(missing)) return;
-  const uint32_t *__restrict__ tab = L.halo_tab;
   const bool fine = sp.is_level_1 == 0;
-  const bool pair = G2 != nullptr;                         // first sub-step of a pair
-  const bool interp = fine && !precomputed;                // this pass interpolates
-  const float tw = sp.temporal_weight;
-  const int gx0 = (mx - 1) * BS + 1, gy0 = (my - 1) * BS + 1, gz0 = (mz - 1) * BS + 1;
-  auto in_domain = [&](int gx, int gy, int gz) {
-    return gx >= 1 && gx <= sp.nx_global && gy >= 1 && gy <= sp.ny_global && gz >= 1 &&
-           gz <= sp.nz_global;
-  };
-  // lists: interface ring positions and slots whose neighbour is absent
-  uint32_t te[kGhostScan];
-#pragma unroll
-  for (int j = 0; j < kGhostScan; ++j) {
-    const int i = t + j * kGhostThreads;
-    te[j] = i < kHaloEntries ? __ldg(tab + i) : 0u;
-  }
-  if (fine) {
-    for (int j = 0; j < (kRingEntries + kGhostThreads - 1) / kGhostThreads; ++j) {
-      const int q = t + j * kGhostThreads;
-      bool want = false;
-      if (q < kRingEntries) {
-        const int p = (int)__ldg(tab + kHaloEntries + q);
-        const int sx = p % 10 - 1, sy = (p / 10) % 10 - 1, sz = p / 100 - 1;
-        const int ox = sx < 0 ? -1 : (sx > 7 ? 1 : 0);
-        const int oy = sy < 0 ? -1 : (sy > 7 ? 1 : 0);
-        const int oz = sz < 0 ? -1 : (sz > 7 ? 1 : 0);
-        want = nbbase[(ox + 1) + 3 * (oy + 1) + 9 * (oz + 1)] < 0 &&
-               in_domain(gx0 + sx, gy0 + sy, gz0 + sz);
-        iface_of[q] = want;
-      }
-      append_if(interp && want, q, &n_pos, pos_list);
+  const int mx = L.map_x[b], my = L.map_y[b], mz = L.map_z[b];
+  // lowest parent cell (1-based) of the block's stencils per axis and its block
+  const int lx = 4 * (mx - 1) - 1, ly = 4 * (my - 1) - 1, lz = 4 * (mz - 1) - 1;
+  const int bx0 = (max(lx, 1) - 1) / BS, by0 = (max(ly, 1) - 1) / BS, bz0 = (max(lz, 1) - 1) / BS;
+  int work = 0;
+  if (t < 27) {
+    int kd = 0;
+    if (t != 13 && L.nbr[b + L.nbr_stride * t] <= 0) {
+      const int nbx = mx + t % 3 - 1, nby = my + (t / 3) % 3 - 1, nbz = mz + t / 9 - 1;
+      const bool inside = nbx >= 1 && nbx * BS <= sp.nx_global && nby >= 1 &&
+                          nby * BS <= sp.ny_global && nbz >= 1 && nbz * BS <= sp.nz_global;
+      // the second sub-step of a pair finds its coarse-to-fine values set
+      kd = fine && inside ? (precomputed ? 0 : 1) : 2;
     }
+    kind[t] = (int8_t)kd;
+    work = kd != 0;
+  } else if (fine && t >= 32 && t < 40) {
+    const int s = t - 32;
+    const int px = bx0 + (s & 1), py = by0 + ((s >> 1) & 1), pz = bz0 + (s >> 2);
+    int pb = 0;
+    if (px < L.pdim_x && py < L.pdim_y && pz < L.pdim_z)
+      pb = L.pptr[px + L.pdim_x * (py + L.pdim_y * pz)];
+    pbase[s] = pb > 0 ? (int32_t)((L.p_block_offset + pb - 1) * BCELLS) : -1;
+  } else if (t == 64) {
+    n_unit = 0;
   }
+  const uint32_t *__restrict__ tab = L.ghost_units;
+  uint32_t head[kGhostScan];
 #pragma unroll
   for (int j = 0; j < kGhostScan; ++j) {
-    const int i = t + j * kGhostThreads;
-    append_if(i < kHaloEntries && nbbase[(te[j] >> 5) & 31] < 0, i, &n_slot, slot_list);
+    const int u = t + j * kGhostThreads;
+    head[j] = u < kGhostUnits ? __ldg(tab + 4 * u) : 13u << 21;
+  }
+  if (!__syncthreads_or(work)) return;
+  const bool pair = G2 != nullptr;                         // first sub-step of a pair
+  const float tw = sp.temporal_weight;
+  const bool temporal = sp.use_temporal_interp == 1;
+  const bool use_old = temporal && tw < 0.99f;
+  const bool use_new = pair || !use_old || tw != 0.0f;
+  const int gx0 = (mx - 1) * BS + 1, gy0 = (my - 1) * BS + 1, gz0 = (mz - 1) * BS + 1;
+  // a parent value at this sub-step's weight and at the second sub-step's
+  auto blend = [&](float fn, float fo, float &v, float &v2) {
+    v = !use_old ? fn : (tw == 0.0f ? fo : lerp_rn(fo, fn, tw));
+    v2 = temporal ? lerp_rn(fo, fn, kSecondSubstepWeight) : fn;
+  };
+  // parent cell of corner s of the group with pair indices (px, py, pz), -1 absent
+  auto corner = [&](int px, int py, int pz, int s) -> int32_t {
+    const int cx = (s & 1) ? lx + px + 1 : max(1, lx + px);
+    const int cy = (s & 2) ? ly + py + 1 : max(1, ly + py);
+    const int cz = (s & 4) ? lz + pz + 1 : max(1, lz + pz);
+    const int q = ((cx - 1) / BS - bx0) + 2 * ((cy - 1) / BS - by0) + 4 * ((cz - 1) / BS - bz0);
+    const int32_t base = pbase[q];
+    return base < 0 ? -1
+                    : base + ((cx - 1) & 7) + BS * ((cy - 1) & 7) + BS * BS * ((cz - 1) & 7);
+  };
+#pragma unroll
+  for (int j = 0; j < kGhostScan; ++j) {
+    const int u = t + j * kGhostThreads;
+    append_if(kind[head[j] >> 21] != 0, u, &n_unit, unit_list);
+  }
+  // interpolated moments of the interface groups: one (group, moment) per thread
+  if (fine && !precomputed) {
+    for (int j = t; j < 4 * kGhostGroups; j += kGhostThreads) {
+      const int q = j >> 2, m = j & 3;
+      const uint32_t gw = __ldg(tab + 4 * kGhostUnits + q);
+      if (kind[gw >> 8] != 1) continue;
+      const int code = gw & 255;
+      const int px = code % 6, py = (code / 6) % 6, pz = code / 36;
+      const float *pn = ghost_moment_plane(L, m, false);
+      const float *po = ghost_moment_plane(L, m, true);
+      const float none = m == 0 ? 1.0f : 0.0f;
+      float v[8], v2[8];
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const int32_t c = corner(px, py, pz, s);
+        v[s] = v2[s] = none;
+        if (c >= 0) blend(use_new ? pn[c] : 0.0f, use_old ? po[c] : 0.0f, v[s], v2[s]);
+        else if (s > 0) { v[s] = v[0]; v2[s] = v2[0]; }
+      }
+#pragma unroll 1
+      for (int sub = 0; sub < 4; ++sub) {
+        int bits = sub;
+        float wx, wy, wz;
+        ghost_member(px, bits, wx);
+        ghost_member(py, bits, wy);
+        ghost_member(pz, bits, wz);
+        if (bits) break;  // the group has fewer positions
+        rs[m][4 * q + sub] = trilerp(v, wx, wy, wz);
+        if (pair) rs2[m][4 * q + sub] = trilerp(v2, wx, wy, wz);
+      }
+    }
   }
   __syncthreads();
-  if (interp) {
-    for (int j = t; j < n_pos; j += kGhostThreads) {
-      const int q = pos_list[j];
-      const int p = (int)__ldg(tab + kHaloEntries + q);
-      const int sx = p % 10 - 1, sy = (p / 10) % 10 - 1, sz = p / 100 - 1;
-      ParentStencil P;
-      parent_stencil(L, gx0 + sx, gy0 + sy, gz0 + sz, P);
-      float r[4];
-      ghost_moments(L, P, tw, r);
+  for (int j = t; j < n_unit; j += kGhostThreads) {
+    const int u = unit_list[j];
+    const uint4 raw = __ldg((const uint4 *)tab + u);
+    const int k = raw.x & 31, q = (raw.x >> 5) & 255, code = (raw.x >> 13) & 255;
+    const int px = code % 6, py = (code / 6) % 6, pz = code / 36;
+    if (kind[raw.x >> 21] == 1) {
+      const T *po = (const T *)ghost_parent(L, true) + (size_t)k * L.p_dstride;
+      const T *pn = (const T *)ghost_parent(L, false) + (size_t)k * L.p_dstride;
+      float v[8], v2[8];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) rs[i][q] = r[i];
-      if (pair) {
-        ghost_moments(L, P, kSecondSubstepWeight, r);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) rs2[i][q] = r[i];
+      for (int s = 0; s < 8; ++s) {
+        const int32_t c = corner(px, py, pz, s);
+        v[s] = v2[s] = w_of(k);
+        if (c >= 0)
+          blend(use_new ? ST::load(pn, c, k, L.p_inv_scale) : 0.0f,
+                use_old ? ST::load(po, c, k, L.p_inv_scale) : 0.0f, v[s], v2[s]);
+        else if (s > 0) { v[s] = v[0]; v2[s] = v2[0]; }
       }
 #pragma unroll
-      for (int s = 0; s < 8; ++s) cs[s][q] = P.ci[s];
-      ws[0][q] = P.wx; ws[1][q] = P.wy; ws[2][q] = P.wz;
-    }
-    __syncthreads();
-  }
-  for (int j = t; j < n_slot; j += kGhostThreads) {
-    const int i = slot_list[j];
-    const uint32_t e = __ldg(tab + i);
-    const int k = e & 31;
-    const int q = fine ? (int)__ldg(tab + kRingIndexOffset + i) : 0;
-    if (fine && iface_of[q]) {
-      if (precomputed) continue;
-      ParentStencil P;
-#pragma unroll
-      for (int s = 0; s < 8; ++s) P.ci[s] = cs[s][q];
-      P.wx = ws[0][q]; P.wy = ws[1][q]; P.wz = ws[2][q];
-      const float r[4] = {rs[0][q], rs[1][q], rs[2][q], rs[3][q]};
-      if (pair) {
-        const float r2[4] = {rs2[0][q], rs2[1][q], rs2[2][q], rs2[3][q]};
-        float g0, g1;
-        ghost_population_pair(L, k, P, r, r2, ST{}, g0, g1);
-        G[i] = g0;
-        G2[i] = g1;
-      } else {
-        G[i] = ghost_population(L, k, P, r, tw, ST{});
+      for (int h = 0; h < 2; ++h) {  // this sub-step's weight, then the second one's
+        if (h == 1 && !pair) break;
+        float *const out = h ? G2 : G;
+        const float(*const rr)[4 * kGhostGroups] = h ? rs2 : rs;
+#pragma unroll 1
+        for (int sub = 0; sub < 4; ++sub) {
+          const uint32_t slot = ((sub < 2 ? raw.y : raw.z) >> (16 * (sub & 1))) & 0xFFFFu;
+          if (slot == kGhostNoSlot) continue;
+          int bits = sub;
+          float wx, wy, wz;
+          ghost_member(px, bits, wx);
+          ghost_member(py, bits, wy);
+          ghost_member(pz, bits, wz);
+          const int i = 4 * q + sub;
+          const float r[4] = {rr[0][i], rr[1][i], rr[2][i], rr[3][i]};
+          out[slot] = ghost_finish(L, k, h ? v2 : v, wx, wy, wz, r);
+        }
       }
     } else {
-      const int p = e >> 19;
-      const int sx = p % 10 - 1, sy = (p / 10) % 10 - 1, sz = p / 100 - 1;
-      G[i] = ghost_boundary(L, k, b, sx + cx_of(k), sy + cy_of(k), sz + cz_of(k), ST{});
+      for (int sub = 0; sub < 4; ++sub) {
+        const uint32_t slot = ((sub < 2 ? raw.y : raw.z) >> (16 * (sub & 1))) & 0xFFFFu;
+        if (slot == kGhostNoSlot) continue;
+        int bits = sub;
+        float w;
+        const int sx = ghost_member(px, bits, w), sy = ghost_member(py, bits, w),
+                  sz = ghost_member(pz, bits, w);
+        const int gx = gx0 + sx, gy = gy0 + sy, gz = gz0 + sz;
+        if (fine && gx >= 1 && gx <= sp.nx_global && gy >= 1 && gy <= sp.ny_global && gz >= 1 &&
+            gz <= sp.nz_global) {
+          if (precomputed) continue;
+          G[slot] = ghost_slot<ST>(L, k, gx, gy, gz, tw);
+          if (pair) G2[slot] = ghost_slot<ST>(L, k, gx, gy, gz, kSecondSubstepWeight);
+        } else {
+          G[slot] = ghost_boundary(L, k, b, sx + cx_of(k), sy + cy_of(k), sz + cz_of(k), ST{});
+        }
+      }
     }
   }
 }

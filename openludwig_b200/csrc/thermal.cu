@@ -124,7 +124,8 @@ extern "C" int ol_thermal(const ol_thermal_view *tv, const ol_thermal_params *tp
                "ol_thermal: OL_GHOST_PAIR_SECOND needs temporal weight 1/2");
   D.tp = *tp;
   D.halo_tab = halo_table_device();
-  if (!D.halo_tab) return set_error(OL_ERR_CUDA, "ol_thermal: staging table allocation failed");
+  D.ghost_units = ghost_units_device();
+  if (!D.halo_tab || !D.ghost_units) return set_error(OL_ERR_CUDA, "ol_thermal: staging table allocation failed");
   if (!tp->is_level_1) {
     OL_CHECK_ARG(tv->pg && tv->pT && tv->pvel && tv->p_block_ptr && tv->p_n_blocks > 0,
                  "ol_thermal: fine level needs parent thermal state");

@@ -20,6 +20,7 @@ struct ThermalDev {
   float p_inv_scale;
   ol_thermal_params tp;
   const uint32_t *halo_tab;
+  const uint32_t *ghost_units;  // unit table of the ghost pass
   float *ghost;            // absent-neighbour pull sources, kHaloEntries per row, or null
   const int32_t *gidx;     // block -> ghost row (-1: none); null = row b for block b
   float *ghost_next;       // as LevelDev::ghost_next / ghost_mode
@@ -78,9 +79,10 @@ __device__ __forceinline__ void ghost_moments(const ThermalDev &D, const ParentS
 
 // g_eq(T, u) + (g - g_eq) * clamp(...) from the 8 corner values of g_k.
 __device__ __forceinline__ float finish_thermal(const ThermalDev &D, int k, const float (&v)[8],
-                                                const ParentStencil &P, const float (&r)[4]) {
+                                                float wx, float wy, float wz,
+                                                const float (&r)[4]) {
   const ol_thermal_params &tp = D.tp;
-  const float gi = trilerp(v, P.wx, P.wy, P.wz);
+  const float gi = trilerp(v, wx, wy, wz);
   const float ge = geq(r[0], r[1], r[2], r[3], w_of(k), (float)cx_of(k), (float)cy_of(k),
                        (float)cz_of(k));
   const float gneq = gi - ge;
@@ -110,37 +112,20 @@ __device__ __forceinline__ float ghost_population(const ThermalDev &D, int k,
 #pragma unroll
   for (int s = 1; s < 8; ++s)
     if (P.ci[s] < 0) v[s] = v[0];
-  return finish_thermal(D, k, v, P, r);
+  return finish_thermal(D, k, v, P.wx, P.wy, P.wz, r);
 }
 
-// Both child sub-steps of a parent step from one read of the parent's old
-// and new g (as interp_population_pair for the flow).
-template <class ST>
-__device__ __forceinline__ void ghost_population_pair(const ThermalDev &D, int k,
-                                                      const ParentStencil &P,
-                                                      const float (&r0)[4], const float (&r1)[4],
-                                                      ST, float &g0, float &g1) {
-  const bool temporal = D.tp.use_temporal_interp == 1;
-  using T = typename ST::T;
-  const T *po = (const T *)D.pg_old + (size_t)k * D.p_dstride;   // plane k
-  const T *pn = (const T *)D.pg + (size_t)k * D.p_dstride;
-  float v0[8], v1[8];
-#pragma unroll
-  for (int s = 0; s < 8; ++s) {
-    v0[s] = v1[s] = w_of(k);
-    if (P.ci[s] >= 0) {
-      const uint32_t c = (uint32_t)P.ci[s];
-      const float gn = ST::load(pn, c, k, D.p_inv_scale);
-      const float go = temporal ? ST::load(po, c, k, D.p_inv_scale) : gn;
-      v0[s] = go;
-      v1[s] = temporal ? lerp_rn(go, gn, kSecondSubstepWeight) : gn;
-    }
-  }
-#pragma unroll
-  for (int s = 1; s < 8; ++s)
-    if (P.ci[s] < 0) { v0[s] = v0[0]; v1[s] = v1[0]; }
-  g0 = finish_thermal(D, k, v0, P, r0);
-  g1 = finish_thermal(D, k, v1, P, r1);
+// The ghost pass's view of the thermal level (stream_collide.cuh).
+__device__ __forceinline__ const float *ghost_moment_plane(const ThermalDev &D, int m, bool old) {
+  if (m == 0) return old ? D.pT_old : D.pT;
+  return (old ? D.pvel_old : D.pvel) + (size_t)(m - 1) * D.p_dstride;
+}
+__device__ __forceinline__ const void *ghost_parent(const ThermalDev &D, bool old) {
+  return old ? D.pg_old : D.pg;
+}
+__device__ __forceinline__ float ghost_finish(const ThermalDev &D, int k, const float (&v)[8],
+                                              float wx, float wy, float wz, const float (&r)[4]) {
+  return finish_thermal(D, k, v, wx, wy, wz, r);
 }
 
 template <class ST>
