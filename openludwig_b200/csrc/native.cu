@@ -563,17 +563,15 @@ static int shape_for(const ol_ctx *c, const Launch &l) {
 
 template <int OP, class ST, bool WALE, bool DDF>
 static void launch_variant(ol_ctx *c, const Launch &l) {
-  if constexpr (OP == OL_OP_CUMULANT && !DDF) {
-    // by default FP32 only: with FP16-shifted storage the warp-specialised
-    // kernel measured slower than one CTA per item (its consumers decode
-    // every landed value)
+  if constexpr (OP == OL_OP_CUMULANT && !DDF && std::is_same<ST, StoreF32>::value) {
+    // FP32 storage only (FP16-shifted populations measured slower this way:
+    // the consumers had to decode every landed value)
     const int choice = stream_collide_kernel_choice();
-    const bool f32 = std::is_same<ST, StoreF32>::value;
     if (choice == OL_SC_KERNEL_WS ||
-        (f32 && shape_for(c, l) == kGridWs && choice == OL_SC_KERNEL_AUTO)) {
+        (shape_for(c, l) == kGridWs && choice == OL_SC_KERNEL_AUTO)) {
       const int grid = ws_grid(l.n, c->n_sm);
-      k_sc_ws<OP, ST, WALE, true><<<(unsigned)grid, kWsThreads, ws_smem_bytes<ST>(), c->stream>>>(
-          LevelDev{}, c->d_descs, c->d_items + l.off, (int)l.n, ws_table_device(),
+      k_sc_ws<OP, WALE, true><<<(unsigned)grid, kWsThreads, kWsBytes, c->stream>>>(
+          LevelDev{}, c->d_descs, c->d_items + l.off, (int)l.n, ws_loader_device(),
           fault_word_device());
       return;
     }
@@ -880,15 +878,9 @@ static int prepare_attributes() {
   cudaFuncSetAttribute(k_sc_pipe<1, true, true>, (cudaFuncAttribute)a, kPipeBytes);
   prepare_attributes_st<StoreF32>();
   prepare_attributes_st<StoreF16S>();
-  cudaFuncSetAttribute(k_sc_ws<0, StoreF32, false, true>, (cudaFuncAttribute)a,
-                       ws_smem_bytes<StoreF32>());
-  cudaFuncSetAttribute(k_sc_ws<0, StoreF32, true, true>, (cudaFuncAttribute)a,
-                       ws_smem_bytes<StoreF32>());
-  cudaFuncSetAttribute(k_sc_ws<0, StoreF16S, false, true>, (cudaFuncAttribute)a,
-                       ws_smem_bytes<StoreF16S>());
-  cudaFuncSetAttribute(k_sc_ws<0, StoreF16S, true, true>, (cudaFuncAttribute)a,
-                       ws_smem_bytes<StoreF16S>());
-  if (!fault_word_device() || !ws_table_device())
+  cudaFuncSetAttribute(k_sc_ws<0, false, true>, (cudaFuncAttribute)a, kWsBytes);
+  cudaFuncSetAttribute(k_sc_ws<0, true, true>, (cudaFuncAttribute)a, kWsBytes);
+  if (!fault_word_device() || !ws_loader_device())
     return set_error(OL_ERR_CUDA, "warp-specialised kernel tables: allocation failed");
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? OL_OK : cuda_status(e, "cudaFuncSetAttribute");

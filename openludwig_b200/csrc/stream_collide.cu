@@ -162,10 +162,25 @@ static std::vector<uint32_t> build_ws_table() {
   return tab;
 }
 
-const uint32_t *ws_table_device() {
+// The same pulls as the kernels read them (ws.cuh): those from the z face
+// neighbours last, whose sources come by bulk copy where the neighbour exists.
+static std::vector<uint32_t> build_ws_loader() {
+  const std::vector<uint32_t> ws = build_ws_table();
+  std::vector<uint32_t> tab;
+  for (int part = 0; part < 3; ++part)
+    for (int i = 0; i < kHaloEntries; ++i) {
+      const uint32_t e = ws[i], k = e & 31, dir = (e >> 5) & 31, src = (e >> 10) & 511;
+      if ((dir == kDirZlo ? 1 : dir == kDirZhi ? 2 : 0) != part) continue;
+      tab.push_back(src | k << 9);
+      tab.push_back(dir | ws[kWsSlotOffset + i] << 5 | (uint32_t)i << 20);
+    }
+  return tab;
+}
+
+const uint32_t *ws_loader_device() {
   static std::mutex mu;
   static uint32_t *per_dev[64] = {};
-  return table_on_device<kWsTableTotal>(per_dev, mu, build_ws_table);
+  return table_on_device<kWsLoaderWords>(per_dev, mu, build_ws_loader);
 }
 
 // Per-device fault word of the warp-specialised kernels (bits kWsFault*):
@@ -254,17 +269,17 @@ static void launch_one(const LevelDev &L0, cudaStream_t s) {
 
 // Warp-specialised persistent kernel over the level's blocks: one CTA per
 // SM (or per block when the level is smaller).
-template <int OP, class ST, bool WALE>
+template <int OP, bool WALE>
 static void launch_ws(const LevelDev &L, int n_sm, cudaStream_t s) {
   static bool done = false;
   if (!done) {
-    cudaFuncSetAttribute(k_sc_ws<OP, ST, WALE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         ws_smem_bytes<ST>());
+    cudaFuncSetAttribute(k_sc_ws<OP, WALE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         kWsBytes);
     done = true;
   }
   const int grid = ws_grid(L.n_blocks, n_sm);
-  launch_pdl(k_sc_ws<OP, ST, WALE, false>, grid, kWsThreads, ws_smem_bytes<ST>(), s, L,
-             (const LevelDev *)nullptr, (const WorkItem *)nullptr, 0, ws_table_device(),
+  launch_pdl(k_sc_ws<OP, WALE, false>, grid, kWsThreads, kWsBytes, s, L,
+             (const LevelDev *)nullptr, (const WorkItem *)nullptr, 0, ws_loader_device(),
              fault_word_device());
 }
 
@@ -292,7 +307,7 @@ static bool ws_applies(const LevelDev &L) {
   if (!a16(L.f_in) || !a16(L.obstacle) || !a16(L.sponge)) return false;
   if (L.sp.c_wale != 0.0f && !a16(L.vel_in)) return false;
   if (L.sp.wall_model_active == 1 && L.wall_dist && !a16(L.wall_dist)) return false;
-  return fault_word_device() != nullptr && ws_table_device() != nullptr;
+  return fault_word_device() != nullptr && ws_loader_device() != nullptr;
 }
 
 template <int OP, bool WALE>
@@ -316,12 +331,12 @@ template <class ST>
 static void launch_sc(const LevelDev &L, cudaStream_t s) {
   const bool wale = L.sp.c_wale != 0.0f;
   const int n_sm = device_sm_count();
-  const bool ws = g_sc_kernel == OL_SC_KERNEL_WS ||
-                  (g_sc_kernel == OL_SC_KERNEL_AUTO && L.n_blocks >= 2 * n_sm &&
-                   std::is_same<ST, StoreF32>::value);
+  const bool ws = std::is_same<ST, StoreF32>::value &&
+                  (g_sc_kernel == OL_SC_KERNEL_WS ||
+                   (g_sc_kernel == OL_SC_KERNEL_AUTO && L.n_blocks >= 2 * n_sm));
   if (ws && ws_applies(L)) {
-    if (wale) launch_ws<OL_OP_CUMULANT, ST, true>(L, n_sm, s);
-    else launch_ws<OL_OP_CUMULANT, ST, false>(L, n_sm, s);
+    if (wale) launch_ws<OL_OP_CUMULANT, true>(L, n_sm, s);
+    else launch_ws<OL_OP_CUMULANT, false>(L, n_sm, s);
     return;
   }
   if (L.sp.op == OL_OP_CUMULANT) {

@@ -1177,12 +1177,12 @@ __device__ __forceinline__ void load_pulls(const float *E, int t, float (&A)[27]
     A[k] = E[k * EPL + eb - (cx_of(k) + 10 * cy_of(k) + 100 * cz_of(k))];
 }
 
-// Per-cell inputs a caller may have read ahead of the collision (the
-// warp-specialised kernel issues them before its shared-memory pulls):
-// the wall distance and the WALE neighbour velocities.
+// Per-cell inputs a caller may have evaluated ahead of the collision (the
+// warp-specialised kernel does so before its shared-memory pulls): the wall
+// distance and the WALE eddy viscosity.
 struct CellAux {
   float wall_dist;
-  WaleVel wale;
+  float nu_wale;
 };
 
 // collide_cell's stores: populations (and the optional post-collision copy)
@@ -1317,7 +1317,7 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
   out.macro(rho, ux, uy, uz);
 
   float nu_eddy = 0.0f;
-  if (WALE) nu_eddy = aux ? wale_from(aux->wale, sp.c_wale) : wale_nu(L, nbbase, x, y, z);
+  if (WALE) nu_eddy = aux ? aux->nu_wale : wale_nu(L, nbbase, x, y, z);
   nu_eddy = fmaxf(nu_eddy, sp.nu_sgs_background);
 
   float omega;  // omega_1 (cumulant) or omega (BGK)

@@ -52,7 +52,7 @@ static bool thermal_ws_applies(const ThermalDev &D, int n_sm) {
     return false;
   if (!D.tp.is_level_1 && !D.ghost) return false;
   if (!a16(D.g_in) || !a16(D.vel) || !a16(D.sponge) || !a16(D.obstacle)) return false;
-  return fault_word_device() != nullptr && ws_table_device() != nullptr;
+  return fault_word_device() != nullptr && ws_loader_device() != nullptr;
 }
 
 template <class ST>
@@ -68,7 +68,7 @@ static void launch_t(const ThermalDev &D, cudaStream_t s) {
   if (D.ghost && gn > 0) k_ghost_fill_thermal<ST><<<gn, kGhostThreads, 0, s>>>(D);
   const int n_sm = sm_count();
   if (std::is_same<ST, StoreF32>::value && thermal_ws_applies(D, n_sm)) {
-    k_thermal_ws<<<ws_grid(D.n_blocks, n_sm), kWsThreads, kTwBytes, s>>>(D, ws_table_device(),
+    k_thermal_ws<<<ws_grid(D.n_blocks, n_sm), kWsThreads, kTwBytes, s>>>(D, ws_loader_device(),
                                                                          fault_word_device());
     return;
   }

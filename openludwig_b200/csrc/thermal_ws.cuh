@@ -31,20 +31,21 @@ constexpr int kTwLdV = kTwS + 27 * kSPlane * 4;        // float [3][512] flow ve
 constexpr int kTwLdSP = kTwLdV + 3 * BCELLS * 4;       // float [512]
 constexpr int kTwLdOB = kTwLdSP + BCELLS * 4;          // uint8 [512]
 constexpr int kTwBuf = kTwLdOB + BCELLS;               // bytes per buffer (79,552)
-constexpr int kTwTab = 2 * kTwBuf;                     // uint32 [kWsTableTotal]
-constexpr int kTwBytes = kTwTab + kWsTableTotal * 4;   // 186,048
+constexpr int kTwTab = 2 * kTwBuf;                     // uint2 [kHaloEntries]
+constexpr int kTwBytes = kTwTab + kWsLoaderWords * 4;  // 184,512
 constexpr int kTwRing = 8;                             // descriptor slots (block j uses j & 7)
 static_assert(kTwLdV % 16 == 0 && kTwLdSP % 16 == 0 && kTwLdOB % 16 == 0 && kTwBuf % 16 == 0,
               "bulk-copy destinations stay 16-byte aligned");
 
 // The producer's bulk copies of block b into the stage (lane 0 announces the
 // bytes, then arrives).
-__device__ __forceinline__ void tws_produce(const ThermalDev &D, int b, int lane,
+__device__ __forceinline__ void tws_produce(const ThermalDev &D, int b, const int *nb, int lane,
                                             unsigned char *sm, uint64_t *bar) {
   constexpr uint32_t kPlane = BCELLS * 4;
   const int64_t own0 = (D.block_offset + b) * BCELLS;
   const float *gin = (const float *)D.g_in;
-  if (lane == 0) mbar_expect_tx(bar, 27 * kPlane + 3 * kPlane + kPlane + BCELLS);
+  const uint32_t layers = 9 * 256 * ((nb[kDirZlo] >= 0) + (nb[kDirZhi] >= 0));
+  if (lane == 0) mbar_expect_tx(bar, 27 * kPlane + 3 * kPlane + kPlane + BCELLS + layers);
   __syncwarp();
   const int c = lane;  // 32 copies, one per lane
   if (c < 27) {
@@ -58,26 +59,7 @@ __device__ __forceinline__ void tws_produce(const ThermalDev &D, int b, int lane
   } else {
     bulk_copy(sm + kTwLdOB, D.obstacle + own0, BCELLS, bar);
   }
-}
-
-// Out-of-block pull sources of consumer thread t (loader-table entries
-// t + 512 m) for block b, into registers.
-__device__ __forceinline__ void tws_halo_load(const ThermalDev &D, int b, const int *nbbase,
-                                              int t, const uint32_t *tabs,
-                                              float (&h)[kWsHaloPerConsumer]) {
-  const float *gin = (const float *)D.g_in;
-  const float *ghost_row = ghost_row_of(D, b);
-#pragma unroll
-  for (int m = 0; m < kWsHaloPerConsumer; ++m) {
-    const int i = t + BCELLS * m;
-    h[m] = 0.0f;
-    if (i >= kHaloEntries) continue;
-    const uint32_t e = tabs[i];
-    const int k = e & 31, dir = (e >> 5) & 31, src = (e >> 10) & 511;
-    const int nb = nbbase[dir];
-    if (nb >= 0) h[m] = __ldg(gin + (size_t)k * D.dstride + nb + src);
-    else if (ghost_row) h[m] = ghost_row[i];
-  }
+  ws_copy_zlayers(gin, D.dstride, nb, lane, (float *)(sm + kTwS), bar);
 }
 
 // The BGK update of cell t from its 27 pulled values A (thermal_cell's
@@ -144,12 +126,13 @@ __global__ void __launch_bounds__(kWsThreads, 1)
   // consumers may still be finishing block j-3
   __shared__ int nbb[kTwRing][27];
   __shared__ int blk[kTwRing];
+  __shared__ int absent[kTwRing];  // some neighbour of the block is absent
   // per buffer: "landed" (bulk bytes plus the producer's arrival), "free"
   // (one arrival per consumer warp); block j uses buffer j & 1, and its
   // (j >> 1)-th phase of each
   __shared__ __align__(8) uint64_t bars[4];
   uint64_t *const landed = &bars[0], *const lfree = &bars[2];
-  uint32_t *const tabs = (uint32_t *)(tw_smem + kTwTab);
+  uint2 *const tabs = (uint2 *)(tw_smem + kTwTab);
   const int t = threadIdx.x;
   const int n = D.n_blocks;
   const int first = blockIdx.x;
@@ -161,7 +144,8 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int i = t; i < kWsTableTotal; i += kWsThreads) tabs[i] = __ldg(tab + i);
+  const bool wide = ws_wide(D.dstride);
+  ws_load_table(tabs, tab, D.dstride, t);
   __syncthreads();
 
   if (t >= BCELLS) {
@@ -170,11 +154,16 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     auto fetch = [&](int p) {
       const int r = p & (kTwRing - 1);
       const int b = first + p * (int)gridDim.x;
+      int nb = 1;
       if (lane < 27) {
-        const int nb = D.nbr[b + D.nbr_stride * lane];
+        nb = D.nbr[b + D.nbr_stride * lane];
         nbb[r][lane] = nb > 0 ? (int)((D.block_offset + nb - 1) * BCELLS) : -1;
       }
-      if (lane == 0) blk[r] = b;
+      const bool miss = __any_sync(0xffffffffu, nb <= 0);
+      if (lane == 0) {
+        blk[r] = b;
+        absent[r] = miss;
+      }
       __syncwarp();
     };
     fetch(0);
@@ -188,7 +177,7 @@ __global__ void __launch_bounds__(kWsThreads, 1)
           j < 2 || mbar_wait(lfree + bi, ((j - 2) >> 1) & 1, fault, kWsFaultLoaderWait);
       if (!__all_sync(0xffffffffu, ok)) break;
       if (j >= 2) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      tws_produce(D, blk[r], lane, tw_smem + bi * kTwBuf, landed + bi);
+      tws_produce(D, blk[r], nbb[r], lane, tw_smem + bi * kTwBuf, landed + bi);
     }
     // bulk copies still in flight (a loop left early) land before the CTA exits
     if (j < cnt)
@@ -198,33 +187,33 @@ __global__ void __launch_bounds__(kWsThreads, 1)
   }
 
   // -------------------------------------------------------------- consumers
-  float h[kWsHaloPerConsumer];
+  HaloRegs h;
+  auto load = [&](int p) {
+    const int r = p & (kTwRing - 1);
+    ws_halo_load((const float *)D.g_in, D.dstride, wide, ghost_row_of(D, blk[r]), nbb[r], t, tabs,
+                 h);
+  };
   for (int j = 0; j < cnt; ++j) {
     const int r = j & (kTwRing - 1), bi = j & 1;
     unsigned char *const buf = tw_smem + bi * kTwBuf;
     float *const F = (float *)(buf + kTwS);
     const bool ok = mbar_wait(landed + bi, (j >> 1) & 1, fault, kWsFaultConsumerWait);
-    if (!consumer_sync_and(ok)) break;  // also: every consumer is done pulling block j-1
     const int *nbase = nbb[r];
     const int b = blk[r];
-    if (j == 0) tws_halo_load(D, b, nbase, t, tabs, h);
-    const bool ghost = ghost_row_of(D, b) != nullptr;
-#pragma unroll
-    for (int m = 0; m < kWsHaloPerConsumer; ++m) {
-      const int i = t + BCELLS * m;
-      if (i >= kHaloEntries) continue;
-      const uint32_t e = tabs[i];
-      const int k = e & 31, dir = (e >> 5) & 31, d = e >> 19;
-      const float v = (nbase[dir] >= 0 || ghost)
-                          ? h[m]
-                          : pull_boundary_thermal<StoreF32>(D, k, b, d & 7, (d >> 3) & 7, d >> 6);
-      F[tabs[kWsSlotOffset + i]] = v;
+    float ux = 0.0f, uy = 0.0f, uz = 0.0f, spg = 0.0f;
+    bool obs = false;
+    if (ok) {
+      if (j == 0) load(0);
+      ws_halo_store(F, nbase, t, tabs, h, absent[r] && !ghost_row_of(D, b),
+                    [&](int k, int x, int y, int z) {
+                      return pull_boundary_thermal<StoreF32>(D, k, b, x, y, z);
+                    });
+      const float *const lv = (const float *)(buf + kTwLdV);
+      ux = lv[t]; uy = lv[BCELLS + t]; uz = lv[2 * BCELLS + t];
+      spg = ((const float *)(buf + kTwLdSP))[t];
+      obs = buf[kTwLdOB + t] != 0;
     }
-    const float *const lv = (const float *)(buf + kTwLdV);
-    const float ux = lv[t], uy = lv[BCELLS + t], uz = lv[2 * BCELLS + t];
-    const float spg = ((const float *)(buf + kTwLdSP))[t];
-    const bool obs = buf[kTwLdOB + t] != 0;
-    consumer_sync();  // the stage holds block j
+    if (!consumer_sync_and(ok)) break;  // the stage holds block j
     float A[27];
 #pragma unroll
     for (int k = 0; k < 27; ++k) A[k] = F[k * kSPlane + kSPad + t - cx_of(k)];
@@ -232,10 +221,7 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if ((t & 31) == 0) mbar_arrive(lfree + bi);
-    if (j + 1 < cnt) {
-      const int r1 = (j + 1) & (kTwRing - 1);
-      tws_halo_load(D, blk[r1], nbb[r1], t, tabs, h);
-    }
+    if (j + 1 < cnt) load(j + 1);
     tws_cell(D, (size_t)nbase[13] + t, A, ux, uy, uz, spg, obs);
   }
 }

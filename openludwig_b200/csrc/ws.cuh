@@ -1,46 +1,54 @@
-// Warp-specialised persistent stream-collide (cumulant operator).
+// Warp-specialised persistent stream-collide (FP32 populations).
 //
 // One CTA per SM walks a static share of the work items (blocks of one level
 // for the drop-in entry point, (descriptor, block) items for the block pool).
 // Its 544 threads have two roles:
-//   * 1 producer warp only starts copies.  While the consumers work on item
-//     j it reads the neighbour-table row of item j+2 and, once the landing
-//     buffer is free again, starts the TMA bulk copies (cp.async.bulk,
-//     completion counted in bytes on an mbarrier) of item j+1's contiguous
-//     arrays: 27 population planes, 3 velocity planes, sponge, obstacle, wall
-//     distance -- 66 KB in FP32, moved without registers or request slots.
-//   * 16 consumer warps, one cell per thread, per item: complete the compute
-//     stage -- with FP32 storage the population planes landed in it already,
-//     each shifted so that every pull is one conflict-free shared load at a
-//     compile-time offset (WsLayout); with FP16 storage they decode the
-//     landed block into a "pre-streamed" stage (the value cell d pulls in
-//     direction k at F[k][d]) -- by writing the out-of-block pull sources
-//     each thread loaded for this item one item earlier (a neighbour's value,
-//     the precomputed ghost value, or, without a ghost row, pull_boundary as
-//     in the one-CTA-per-block kernel) into the slots of the cells that pull
-//     them, and the velocities into 10^3 slots per component with a one-cell
-//     face halo (a face without neighbour repeats the cell beside it, the
-//     zero-gradient fallback of the WALE gradients); then pull, release the
-//     buffer the next bulk copies land in, issue the out-of-block loads of
-//     item j+1 into registers, collide and store straight to global memory.
-//     The next item's bulk copies and out-of-block loads land while they
-//     collide.
-// Why this split (measured on B200): a block is 66 KB, and an SM has to keep
-// ~60-90 KB in flight to draw its share of HBM bandwidth.  Loader warps that
-// moved everything themselves -- 4-byte cp.async of every value (too few in
-// flight, 128 bytes each), 16-byte loads through their registers (too few
-// bytes per round trip), bulk copies they then redistributed (four warps
-// cannot hide their own latency), or 4-byte cp.async of just the 3176
-// scattered out-of-block values (still ~15k cycles per block) -- all left
-// the consumers waiting for data more than half the time.
-// Hand-over uses mbarriers ("landed": bulk bytes plus the producer's
-// arrival; "free": one arrival per consumer warp) and a named barrier among
-// the consumers around the stage.  Every mbarrier wait is bounded in time: a
-// wait that runs out sets a bit in the fault word, and the warps give up
-// together (consumers through the same named barriers, the producer after
-// its copies in flight have landed), so no thread is left at a barrier and
-// the kernel always ends.  The staged values are the ones the
-// one-CTA-per-block kernel pulls, and the cell update is the same code.
+//   * 1 producer warp only starts copies.  It reads the neighbour-table row of
+//     item j+1 and, once stage buffer j & 1 is free, starts the TMA bulk copies
+//     (cp.async.bulk, completion counted in bytes on an mbarrier) of item j's
+//     contiguous arrays: 27 population planes, 3 velocity planes, sponge,
+//     obstacle, wall distance, and the 64-cell layers of the two z neighbours
+//     (9 population planes each and their velocities) -- 72 KB, moved without
+//     registers or request slots.
+//   * 16 consumer warps, one cell per thread, per item: write the remaining
+//     out-of-block pull sources, which each thread loaded for this item one
+//     item earlier (a neighbour's value, the precomputed ghost value, or,
+//     without a ghost row, pull_boundary as in the one-CTA-per-block kernel),
+//     into the stage slots of the cells that pull them; barrier; WALE from the
+//     staged velocities; pull; release the buffer; issue the out-of-block
+//     loads of item j+1 into registers; collide and store to global memory.
+//
+// Stage.  Each population plane k lands shifted by 8 c_y + 64 c_z slots in a
+// plane of kSPlane = 72 + 512 + 72 slots, so the value cell t pulls in
+// direction k sits at S[k][t - c_x]: one conflict-free shared load at a
+// compile-time offset.  (The shifts reach 72 cells either way; every landing
+// address stays 32-byte aligned.)  A z neighbour's layer continues its plane
+// on the side the shift left free; the slots whose source lies in the other
+// neighbours are overwritten after the landing.  Velocities: 512 own values,
+// then the 6 x 64 values beyond the faces (a face without a neighbour repeats
+// the cell beside it, the zero-gradient fallback of the WALE gradients).
+//
+// Why this split (measured on B200, cube_3lvl, us per coarse step of this
+// kernel): an SM has to keep ~60-90 KB in flight to draw its share of HBM
+// bandwidth, which bulk copies do and loader warps do not (see the variants in
+// the design notes).  With one stage buffer the next landing could only start
+// after the pulls and end before the next item, so the consumers waited for
+// it: 905 us; with two buffers, z layers by bulk copy and one barrier 766 us
+// (sphere_ddf: 291 -> 260 us, the thermal kernel built the same way 245 -> 222)  Of the 3176 out-of-block
+// sources 968 lie in the z neighbours' contiguous layers and come by bulk copy;
+// the consumers carry the other 2208 (5 registers a thread instead of 7), each
+// found by one 8-byte table entry whose plane offset is formed once per launch.
+//
+// Hand-over uses mbarriers ("landed": bulk bytes plus the producer's arrival;
+// "free": one arrival per consumer warp, both per buffer) and one named barrier
+// of the consumers per item, after the out-of-block values are written.  A
+// buffer lands again only after every consumer has pulled from it, so no
+// barrier is needed before the writes.  Every mbarrier wait is bounded in time:
+// a wait that runs out sets a bit in the fault word, and the warps give up
+// together (consumers through the same named barrier, the producer after its
+// copies in flight have landed), so no thread is left at a barrier and the
+// kernel always ends.  The staged values are the ones the one-CTA-per-block
+// kernel pulls, and the cell update is the same code.
 #pragma once
 #include "stream_collide.cuh"
 
@@ -48,75 +56,51 @@ namespace ol {
 
 constexpr int kWsProducers = 32;                   // 1 producer warp
 constexpr int kWsThreads = BCELLS + kWsProducers;  // 544
-constexpr int kWsRing = 4;  // descriptor / neighbour-offset slots (item j uses j & 3)
-// Table of the warp-specialised kernel: the kHaloEntries out-of-block pulls
-// in the order of the staging table (k | dir << 5 | source cell << 10 |
-// destination cell << 19), then the kWsVelEntries face-halo velocity slots
-// (face dir | own cell beside the slot << 5).
-constexpr int kWsVelEntries = 6 * 64;
-constexpr int kWsTableSize = kHaloEntries + kWsVelEntries;
-// ... then, per out-of-block pull i, the index of the FP32 compute-stage slot
-// it is written to (k * kSPlane + kSPad + destination cell - c_x(k); below)
-constexpr int kWsSlotOffset = kWsTableSize;
-constexpr int kWsTableTotal = kWsTableSize + kHaloEntries;
-// Dynamic shared memory (byte offsets).
-// FP32 storage ("direct"): the bulk copies land each population plane k
-// straight into the compute stage, shifted by 8 c_y + 64 c_z cells, so the
-// value cell t pulls in direction k sits at S[k][t - c_x]: no spread of the
-// landed block, one conflict-free shared load per pull.  A plane of the stage
-// holds 72 + 512 + 72 slots (the shifts reach 72 cells either way; every
-// landing address stays 32-byte aligned); the slots whose source lies
-// outside the block are then overwritten with the out-of-block values.  The
-// stage is the landing buffer, so it is free for the next item once the
-// consumers have pulled.  Velocity, sponge, wall distance and mask land
-// beside it.
-// FP16-shifted storage: the planes land in a buffer of their own and the
-// consumers decode them into a pre-streamed stage F[k][d] (the value cell d
-// pulls in direction k), releasing the buffer before they pull.
+// descriptor / neighbour-offset slots (item j uses j & 7): the producer fetches
+// item j+1 before buffer j & 1 is free, while a consumer may still update j-3
+constexpr int kWsRing = 8;
 constexpr int kSPad = 72;                         // stage slots before cell 0 (and after 511)
 constexpr int kSPlane = kSPad + BCELLS + kSPad;   // 656 floats = 2624 bytes
-template <class ST> struct WsLayout;
-template <> struct WsLayout<StoreF32> {
-  static constexpr bool kDirect = true;
-  static constexpr int kS = 0;                                  // float [27][kSPlane]
-  static constexpr int kV = kS + 27 * kSPlane * 4;              // float [3][1000]
-  static constexpr int kLdV = kV + 3 * EPL * 4;                 // float [3][512]
-  static constexpr int kLdSP = kLdV + 3 * BCELLS * 4;           // float [512]
-  static constexpr int kLdWD = kLdSP + BCELLS * 4;              // float [512]
-  static constexpr int kLdOB = kLdWD + BCELLS * 4;              // uint8 [512]
-  static constexpr int kTab = kLdOB + BCELLS;                   // uint32 [kWsTableTotal]
-  static constexpr int kBytes = kTab + kWsTableTotal * 4;       // 120,544
-  static constexpr int kLdF = 0, kF = 0;                        // (unused)
-};
-template <> struct WsLayout<StoreF16S> {
-  static constexpr bool kDirect = false;
-  static constexpr int kLdF = 0;                                // half [27][512]
-  static constexpr int kLdV = kLdF + 27 * BCELLS * 4;           // float [3][512]
-  static constexpr int kLdSP = kLdV + 3 * BCELLS * 4;           // float [512]
-  static constexpr int kLdWD = kLdSP + BCELLS * 4;              // float [512]
-  static constexpr int kLdOB = kLdWD + BCELLS * 4;              // uint8 [512]
-  static constexpr int kF = kLdOB + BCELLS;                     // float [27][512], pre-streamed
-  static constexpr int kV = kF + 27 * BCELLS * 4;               // float [3][1000]
-  static constexpr int kTab = kV + 3 * EPL * 4;                 // uint32 [kWsTableTotal]
-  static constexpr int kBytes = kTab + kWsTableTotal * 4;       // 160,288
-  static constexpr int kS = 0;                                  // (unused)
-};
-static_assert(WsLayout<StoreF32>::kV % 16 == 0 && WsLayout<StoreF32>::kLdV % 16 == 0 &&
-                  WsLayout<StoreF32>::kLdOB % 16 == 0 && (kSPlane * 4) % 32 == 0 &&
-                  (kSPad * 4) % 32 == 0,
+
+// The table ol_staging_tables exports (kWsTableTotal words): the kHaloEntries
+// out-of-block pulls in the order of the staging table (k | dir << 5 | source
+// cell << 10 | destination cell << 19), the kWsVelEntries face-halo velocity
+// entries (face dir | own cell beside the slot << 5), then per pull its stage
+// slot k * kSPlane + kSPad + destination cell - c_x(k).
+constexpr int kWsVelEntries = 6 * 64;
+constexpr int kWsTableSize = kHaloEntries + kWsVelEntries;
+constexpr int kWsSlotOffset = kWsTableSize;
+constexpr int kWsTableTotal = kWsTableSize + kHaloEntries;
+// The loader table in device memory: two words per pull, {source cell |
+// k << 9, dir | stage slot << 5 | staging-table index << 20}; first the
+// kWsInner pulls the consumers always carry, then the 2 x kWsZFace pulls from
+// the -z and +z face neighbours (carried only where that neighbour is absent).
+constexpr int kWsZFace = 484;
+constexpr int kWsInner = kHaloEntries - 2 * kWsZFace;  // 2208
+constexpr int kWsLoaderWords = 2 * kHaloEntries;
+constexpr int kDirZlo = 4, kDirZhi = 22;
+
+// Dynamic shared memory (bytes): two buffers, then the loader table.
+constexpr int kWsVPlane = BCELLS + kWsVelEntries;             // 896 floats
+constexpr int kWsS = 0;                                       // float [27][kSPlane]
+constexpr int kWsV = kWsS + 27 * kSPlane * 4;                 // float [3][kWsVPlane]
+constexpr int kWsSP = kWsV + 3 * kWsVPlane * 4;               // float [512]
+constexpr int kWsWD = kWsSP + BCELLS * 4;                     // float [512]
+constexpr int kWsOB = kWsWD + BCELLS * 4;                     // uint8 [512]
+constexpr int kWsBuf = kWsOB + BCELLS;                        // 86,208
+constexpr int kWsTab = 2 * kWsBuf;                            // uint2 [kHaloEntries]
+constexpr int kWsBytes = kWsTab + kWsLoaderWords * 4;         // 197,824
+static_assert(kWsV % 16 == 0 && (kWsVPlane * 4) % 16 == 0 && kWsSP % 16 == 0 && kWsOB % 16 == 0 &&
+                  kWsBuf % 16 == 0 && (kSPlane * 4) % 32 == 0 && (kSPad * 4) % 32 == 0,
               "bulk-copy destinations stay 16-byte aligned");
-static_assert(WsLayout<StoreF16S>::kF % 16 == 0 && WsLayout<StoreF16S>::kV % 16 == 0,
-              "alignment");
-template <class ST>
-constexpr int ws_smem_bytes() { return WsLayout<ST>::kBytes; }
-constexpr int kWsHaloPerConsumer = (kHaloEntries + BCELLS - 1) / BCELLS;  // 7
+constexpr int kWsHaloPerConsumer = (kWsInner + BCELLS - 1) / BCELLS;  // 5
 // A wait that has not completed after this long (ns) is treated as lost.
 constexpr unsigned long long kWsWaitNs = 2000000000ull;
 // Bits of the fault word.
 constexpr int kWsFaultConsumerWait = 1, kWsFaultLoaderWait = 2;
 
 // Per-device loader table (built once; null on failure).
-const uint32_t *ws_table_device();
+const uint32_t *ws_loader_device();
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -128,12 +112,6 @@ __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(
                    smem_addr(bar))
-               : "memory");
-}
-// One arrival once every cp.async this thread has issued so far has landed
-// (.noinc: the arrival is part of the barrier's expected count).
-__device__ __forceinline__ void mbar_arrive_cp_async(uint64_t *bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar))
                : "memory");
 }
 __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
@@ -165,24 +143,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *f
   return false;
 }
 
-__device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_4_if(bool p, uint32_t dst, const void *src) {
-  if (p) cp_async_4(dst, src);
-}
-__device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
-// Barrier of the 512 consumer threads only (named barrier 1); the AND form
-// returns whether all of them passed a non-zero predicate.
-__device__ __forceinline__ void consumer_sync() {
-  asm volatile("bar.sync 1, %0;" ::"n"(BCELLS) : "memory");
-}
+// Barrier of the 512 consumer threads only (named barrier 1); returns whether
+// all of them passed a non-zero predicate.
 __device__ __forceinline__ bool consumer_sync_and(int pred) {
   int r;
   asm volatile(
@@ -210,97 +172,177 @@ __device__ __forceinline__ void bulk_copy(void *dst, const void *src, uint32_t b
       : "memory");
 }
 
-// The producer warp's bulk copies of one item into the landing buffer ld
-// (lane 0 announces the bytes, then arrives; the bytes complete the phase).
-template <class ST, bool WALE>
-__device__ __forceinline__ void ws_produce(const LevelDev &L, int b, int lane, unsigned char *ld,
-                                           uint64_t *bar) {
-  using T = typename ST::T;
-  using Lay = WsLayout<ST>;
-  constexpr uint32_t kPlane = BCELLS * sizeof(T);
+// Loader table into shared memory with the plane offsets of this launch:
+// tabs[i] = {k * dstride + source cell (mod 2^32), dir | slot << 5 | index << 20}.
+__device__ __forceinline__ void ws_load_table(uint2 *tabs, const uint32_t *__restrict__ tab,
+                                              int64_t dstride, int t) {
+  for (int i = t; i < kHaloEntries; i += kWsThreads) {
+    const uint2 e = __ldg((const uint2 *)tab + i);
+    tabs[i] = make_uint2((e.x >> 9) * (uint32_t)dstride + (e.x & 511), e.y);
+  }
+}
+// Whether the 27 planes reach beyond 32-bit element offsets (over 159 M cells).
+__device__ __forceinline__ bool ws_wide(int64_t dstride) { return 27 * dstride > 0xFFFFFFFFll; }
+__device__ __forceinline__ int ws_slot(uint2 e) { return (e.y >> 5) & 0x7FFF; }
+// Element offset of entry e's source in the neighbour block whose first cell is nb.
+__device__ __forceinline__ int64_t ws_source(uint2 e, int nb, int64_t dstride, bool wide) {
+  if (!wide) return (int64_t)(e.x + (uint32_t)nb);
+  const int k = ws_slot(e) / kSPlane;
+  return k * dstride + (uint32_t)(e.x - (uint32_t)k * (uint32_t)dstride) + nb;
+}
+
+// The z neighbours' layers of the 9 population planes that pull across that
+// face, by lane 0..8 (-z) and 9..17 (+z), where the neighbour exists.
+__device__ __forceinline__ void ws_copy_zlayers(const float *fin, int64_t dstride, const int *nb,
+                                                int lane, float *S, uint64_t *bar) {
+  if (lane >= 18) return;
+  const bool hi = lane >= 9;
+  const int base = nb[hi ? kDirZhi : kDirZlo];
+  if (base < 0) return;
+  // c_z = +1 pulls across the -z face from the neighbour's z = 7 layer
+  const int k = hi ? lane - 9 : lane + 18;
+  const int at = k * kSPlane + kSPad + 8 * cy_of(k) + (hi ? BCELLS - 64 : 0);
+  bulk_copy(S + at, fin + (size_t)k * dstride + base + (hi ? 0 : BCELLS - 64), 256, bar);
+}
+
+// The producer warp's bulk copies of block b into a buffer (lane 0 announces
+// the bytes, then arrives; the bytes complete the phase).
+template <bool WALE>
+__device__ __forceinline__ void ws_produce(const LevelDev &L, int b, const int *nb, int lane,
+                                           unsigned char *buf, uint64_t *bar) {
+  constexpr uint32_t kPlane = BCELLS * 4;
   const int64_t own0 = (L.block_offset + b) * BCELLS;
   const bool wd = L.sp.wall_model_active == 1 && L.wall_dist;
-  const T *fin = (const T *)L.f_in;
-  const uint32_t bytes = 27 * kPlane + (WALE ? 3 * BCELLS * 4 : 0) + BCELLS * 4 + BCELLS +
-                         (wd ? BCELLS * 4 : 0);
+  const float *fin = (const float *)L.f_in;
+  const uint32_t layers = 9 * 256 * ((nb[kDirZlo] >= 0) + (nb[kDirZhi] >= 0));
+  const uint32_t bytes = 27 * kPlane + layers + (WALE ? 3 * kPlane + 6 * 256 : 0) + kPlane +
+                         BCELLS + (wd ? kPlane : 0);
   if (lane == 0) mbar_expect_tx(bar, bytes);
   __syncwarp();
-  for (int c = lane; c < 33; c += 32) {
-    if (c < 27) {
-      // direct: plane c shifted by 8 c_y + 64 c_z slots (a multiple of 8)
-      unsigned char *dst =
-          Lay::kDirect
-              ? ld + Lay::kS + (c * kSPlane + kSPad + 8 * cy_of(c) + 64 * cz_of(c)) * 4
-              : ld + Lay::kLdF + c * kPlane;
-      bulk_copy(dst, fin + (size_t)c * L.dstride + own0, kPlane, bar);
-    } else if (c < 30) {
-      if (WALE)
-        bulk_copy(ld + Lay::kLdV + (c - 27) * BCELLS * 4,
-                  L.vel_in + (size_t)(c - 27) * L.dstride + own0, BCELLS * 4, bar);
-    } else if (c == 30) {
-      bulk_copy(ld + Lay::kLdSP, L.sponge + own0, BCELLS * 4, bar);
-    } else if (c == 31) {
-      bulk_copy(ld + Lay::kLdOB, L.obstacle + own0, BCELLS, bar);
-    } else if (wd) {
-      bulk_copy(ld + Lay::kLdWD, L.wall_dist + own0, BCELLS * 4, bar);
-    }
+  float *const S = (float *)(buf + kWsS);
+  float *const V = (float *)(buf + kWsV);
+  if (lane < 27) {
+    // plane k = lane shifted by 8 c_y + 64 c_z slots (a multiple of 8)
+    bulk_copy(S + lane * kSPlane + kSPad + 8 * cy_of(lane) + 64 * cz_of(lane),
+              fin + (size_t)lane * L.dstride + own0, kPlane, bar);
+  } else if (lane < 30) {
+    if (WALE)
+      bulk_copy(V + (lane - 27) * kWsVPlane, L.vel_in + (size_t)(lane - 27) * L.dstride + own0,
+                kPlane, bar);
+  } else if (lane == 30) {
+    bulk_copy(buf + kWsSP, L.sponge + own0, kPlane, bar);
+  } else {
+    bulk_copy(buf + kWsOB, L.obstacle + own0, BCELLS, bar);
+    if (wd) bulk_copy(buf + kWsWD, L.wall_dist + own0, kPlane, bar);
+  }
+  ws_copy_zlayers(fin, L.dstride, nb, lane, S, bar);
+  if (WALE && lane >= 18 && lane < 24) {
+    // the velocities beyond the z faces (the own layer where there is no neighbour)
+    const int c = (lane - 18) % 3;
+    const bool hi = lane >= 21;
+    const int base = nb[hi ? kDirZhi : kDirZlo];
+    const int64_t src = base >= 0 ? (int64_t)base + (hi ? 0 : BCELLS - 64)
+                                  : own0 + (hi ? BCELLS - 64 : 0);
+    bulk_copy(V + c * kWsVPlane + BCELLS + (hi ? 320 : 256),
+              L.vel_in + (size_t)c * L.dstride + src, 256, bar);
   }
 }
 
-// Out-of-block pull sources of consumer thread t (table entries t + 512 m)
-// and its face-halo velocities (entry t < 384), loaded into registers.
+// Out-of-block pull sources of consumer thread t (table entries t + 512 m; one
+// per absent z face) into registers.
 struct HaloRegs {
   float f[kWsHaloPerConsumer];
-  float v[3];
+  float z[2];
 };
-template <class ST, bool WALE>
-__device__ __forceinline__ void ws_halo_load(const LevelDev &L, int b, const int *nbbase, int t,
-                                             const uint32_t *tabs, HaloRegs &h) {
-  using T = typename ST::T;
-  const T *fin = (const T *)L.f_in;
-  const float *ghost_row = ghost_row_of(L, b);
+__device__ __forceinline__ void ws_halo_load(const float *__restrict__ fin, int64_t dstride,
+                                             bool wide, const float *__restrict__ ghost_row,
+                                             const int *nb, int t, const uint2 *tabs,
+                                             HaloRegs &h) {
 #pragma unroll
   for (int m = 0; m < kWsHaloPerConsumer; ++m) {
     const int i = t + BCELLS * m;
     h.f[m] = 0.0f;
-    if (i >= kHaloEntries) continue;
-    const uint32_t e = tabs[i];
-    const int k = e & 31, dir = (e >> 5) & 31, src = (e >> 10) & 511;
-    const int nb = nbbase[dir];
-    if (nb >= 0) h.f[m] = ST::load(fin, (size_t)k * L.dstride + nb + src, k, L.inv_scale);
-    else if (ghost_row) h.f[m] = ghost_row[i];
+    if (i >= kWsInner) continue;
+    const uint2 e = tabs[i];
+    const int base = nb[e.y & 31];
+    if (base >= 0) h.f[m] = __ldg(fin + ws_source(e, base, dstride, wide));
+    else if (ghost_row) h.f[m] = __ldg(ghost_row + (e.y >> 20));
   }
-  if (WALE && t < kWsVelEntries) {
-    const uint32_t e = tabs[kHaloEntries + t];
-    const int dir = e & 31, oc = (int)(e >> 5);
-    const int dx = dir % 3 - 1, dy = (dir / 3) % 3 - 1, dz = dir / 9 - 1;
-    const int nb = nbbase[dir];
-    const int64_t src = nb >= 0 ? (int64_t)nb + oc - (7 * dx + 56 * dy + 448 * dz)
-                                : (L.block_offset + b) * BCELLS + oc;
+  h.z[0] = h.z[1] = 0.0f;
+  if (ghost_row && t < kWsZFace) {
+    if (nb[kDirZlo] < 0) h.z[0] = __ldg(ghost_row + (tabs[kWsInner + t].y >> 20));
+    if (nb[kDirZhi] < 0) h.z[1] = __ldg(ghost_row + (tabs[kWsInner + kWsZFace + t].y >> 20));
+  }
+}
+// The same values into the stage.  bc: the block has absent neighbours and no
+// ghost row, so the sources there are evaluated by `boundary(k, x, y, z)`.
+template <class BC>
+__device__ __forceinline__ void ws_halo_store(float *S, const int *nb, int t, const uint2 *tabs,
+                                              const HaloRegs &h, bool bc, BC boundary) {
+  auto eval = [&](uint2 e) {
+    const int slot = ws_slot(e), k = slot / kSPlane;
+    const int d = slot - k * kSPlane - kSPad + cx_of(k);
+    return boundary(k, d & 7, (d >> 3) & 7, d >> 6);
+  };
 #pragma unroll
-    for (int c = 0; c < 3; ++c) h.v[c] = __ldg(L.vel_in + (size_t)c * L.dstride + src);
+  for (int m = 0; m < kWsHaloPerConsumer; ++m) {
+    const int i = t + BCELLS * m;
+    if (i >= kWsInner) continue;
+    const uint2 e = tabs[i];
+    float v = h.f[m];
+    if (bc && nb[e.y & 31] < 0) v = eval(e);
+    S[ws_slot(e)] = v;
+  }
+  if (t < kWsZFace) {
+    if (nb[kDirZlo] < 0) {
+      const uint2 e = tabs[kWsInner + t];
+      S[ws_slot(e)] = bc ? eval(e) : h.z[0];
+    }
+    if (nb[kDirZhi] < 0) {
+      const uint2 e = tabs[kWsInner + kWsZFace + t];
+      S[ws_slot(e)] = bc ? eval(e) : h.z[1];
+    }
   }
 }
 
-// Whether the pull of direction k by cell t + c_k stays in the block.
-struct CellMask {
-  bool xlo, xhi, ylo, yhi, zlo, zhi;  // x > 0, x < 7, y > 0, y < 7, z > 0, z < 7
-};
-__device__ __forceinline__ bool pull_inside(const CellMask &m, int k) {
-  const int cx = cx_of(k), cy = cy_of(k), cz = cz_of(k);
-  return (cx == 0 || (cx > 0 ? m.xhi : m.xlo)) && (cy == 0 || (cy > 0 ? m.yhi : m.ylo)) &&
-         (cz == 0 || (cz > 0 ? m.zhi : m.zlo));
+// Velocities beyond the x and y faces: thread t < 256 holds those of cell
+// t & 63 of face t >> 6 (-x, +x, -y, +y).
+__device__ __forceinline__ void ws_vel_load(const LevelDev &L, int b, const int *nb, int t,
+                                            float (&v)[3]) {
+  if (t >= 256) return;
+  const int face = t >> 6, q = t & 63;
+  const bool yf = face >= 2, hi = face & 1;
+  const int dir = yf ? (hi ? 16 : 10) : (hi ? 14 : 12);
+  const int step = yf ? 56 : 7;  // across the block along the axis
+  const int oc = (yf ? (q & 7) + 64 * (q >> 3) : 8 * q) + (hi ? step : 0);
+  const int base = nb[dir];
+  const int64_t src = base >= 0 ? (int64_t)base + oc + (hi ? -step : step)
+                                : (L.block_offset + b) * BCELLS + oc;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) v[c] = __ldg(L.vel_in + (size_t)c * L.dstride + src);
 }
-__device__ __forceinline__ float land_value(const unsigned char *ld, int k, int c, float inv_scale,
-                                            StoreF16S) {
-  const float w = w_of(k);
-  return fmaf(__half2float(((const __half *)(ld + WsLayout<StoreF16S>::kLdF))[k * BCELLS + c]),
-              w * inv_scale, w);
+// WALE eddy viscosity of cell t from the staged velocities.
+__device__ __forceinline__ float ws_wale(const float *V, int t, float c_wale) {
+  const int x = t & 7, y = (t >> 3) & 7, z = t >> 6;
+  const float *const H = V + BCELLS;
+  const int yz = y + 8 * z, xz = x + 8 * z, xy = x + 8 * y;
+  const float *const pe = x < 7 ? V + t + 1 : H + 64 + yz;
+  const float *const pw = x > 0 ? V + t - 1 : H + yz;
+  const float *const pn = y < 7 ? V + t + 8 : H + 192 + xz;
+  const float *const ps = y > 0 ? V + t - 8 : H + 128 + xz;
+  const float *const pt = z < 7 ? V + t + 64 : H + 320 + xy;
+  const float *const pb = z > 0 ? V + t - 64 : H + 256 + xy;
+  WaleVel w;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    w.e[c] = pe[c * kWsVPlane]; w.w[c] = pw[c * kWsVPlane];
+    w.n[c] = pn[c * kWsVPlane]; w.s[c] = ps[c * kWsVPlane];
+    w.t[c] = pt[c * kWsVPlane]; w.b[c] = pb[c * kWsVPlane];
+  }
+  return wale_from(w, c_wale);
 }
-__device__ __forceinline__ float land_value(const unsigned char *, int, int, float, StoreF32) {
-  return 0.0f;  // (direct layout: no spread)
-}
-template <int OP, class ST, bool WALE, bool BATCHED>
+
+template <int OP, bool WALE, bool BATCHED>
 __global__ void __launch_bounds__(kWsThreads, 1)
     k_sc_ws(const __grid_constant__ LevelDev L0, const LevelDev *__restrict__ descs,
             const WorkItem *__restrict__ items, int n_items, const uint32_t *__restrict__ tab,
@@ -309,28 +351,33 @@ __global__ void __launch_bounds__(kWsThreads, 1)
   __shared__ __align__(16) LevelDev Ls[BATCHED ? kWsRing : 1];
   __shared__ int nbb[kWsRing][27];
   __shared__ int blk[kWsRing];
-  __shared__ __align__(8) uint64_t bars[2];  // landed, free
-  uint64_t *const landed = &bars[0], *const lfree = &bars[1];
-  unsigned char *const ld = ws_smem;
-  using Lay = WsLayout<ST>;
-  uint32_t *const tabs = (uint32_t *)(ws_smem + Lay::kTab);
+  __shared__ const float *grow[kWsRing];  // the item's ghost row (null: none)
+  __shared__ int absent[kWsRing];         // some neighbour of the item is absent
+  __shared__ __align__(8) uint64_t bars[4];
+  uint64_t *const landed = &bars[0], *const lfree = &bars[2];
+  uint2 *const tabs = (uint2 *)(ws_smem + kWsTab);
   const int t = threadIdx.x;
   const int n = BATCHED ? n_items : L0.n_blocks;
   const int first = blockIdx.x;
   const int cnt = first < n ? (n - 1 - first) / (int)gridDim.x + 1 : 0;
+  // every descriptor of a pool has the pool's plane stride
+  const int64_t dstride = BATCHED ? descs[items[first].desc].dstride : L0.dstride;
+  const bool wide = ws_wide(dstride);
   if (t == 0) {
-    mbar_init(landed, 1);          // the producer's expect_tx arrival + the bulk bytes
-    mbar_init(lfree, BCELLS / 32);  // one arrival per consumer warp
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(landed + i, 1);            // the producer's expect_tx arrival + the bulk bytes
+      mbar_init(lfree + i, BCELLS / 32);   // one arrival per consumer warp
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int i = t; i < kWsTableTotal; i += kWsThreads) tabs[i] = __ldg(tab + i);
+  ws_load_table(tabs, tab, dstride, t);
   __syncthreads();
   pdl_wait();  // f_in, vel_in, ghost rows: written by the launches before this one
 
   if (t >= BCELLS) {
     // ------------------------------------------------------------ producer
     const int lane = t - BCELLS;
-    // descriptor and neighbour offsets of item p into ring slot p & 3
+    // descriptor and neighbour offsets of item p into ring slot p & 7
     auto fetch = [&](int p) {
       const int r = p & (kWsRing - 1);
       const int it = first + p * (int)gridDim.x;
@@ -344,11 +391,17 @@ __global__ void __launch_bounds__(kWsThreads, 1)
         __syncwarp();
       }
       const LevelDev &L = BATCHED ? Ls[r] : L0;
+      int nb = 1;
       if (lane < 27) {
-        const int nb = L.nbr[b + L.nbr_stride * lane];
+        nb = L.nbr[b + L.nbr_stride * lane];
         nbb[r][lane] = nb > 0 ? (int)((L.block_offset + nb - 1) * BCELLS) : -1;
       }
-      if (lane == 0) blk[r] = b;
+      const bool miss = __any_sync(0xffffffffu, nb <= 0);
+      if (lane == 0) {
+        blk[r] = b;
+        absent[r] = miss;
+        grow[r] = miss ? ghost_row_of(L, b) : nullptr;
+      }
       __syncwarp();
     };
     // item 0's and item 1's offsets are published with item 0's copies;
@@ -357,114 +410,70 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     if (cnt > 1) fetch(1);
     int j = 0;
     for (; j < cnt; ++j) {
-      const int r = j & (kWsRing - 1);
+      const int r = j & (kWsRing - 1), bi = j & 1;
       if (j >= 1 && j + 1 < cnt) fetch(j + 1);
-      // the landing buffer is free once the consumers have spread item j-1
-      const bool ok = j == 0 || mbar_wait(lfree, (j - 1) & 1, fault, kWsFaultLoaderWait);
+      // buffer bi is free once the consumers have pulled item j-2
+      const bool ok =
+          j < 2 || mbar_wait(lfree + bi, ((j - 2) >> 1) & 1, fault, kWsFaultLoaderWait);
       if (!__all_sync(0xffffffffu, ok)) break;
-      if (j > 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      const LevelDev &L = BATCHED ? Ls[r] : L0;
-      ws_produce<ST, WALE>(L, blk[r], lane, ld, landed);
+      if (j >= 2) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      ws_produce<WALE>(BATCHED ? Ls[r] : L0, blk[r], nbb[r], lane, ws_smem + bi * kWsBuf,
+                       landed + bi);
     }
     // bulk copies still in flight (a loop left early) land before the CTA exits
-    if (j > 0 && j < cnt) mbar_wait(landed, (j - 1) & 1, nullptr, 0);
+    if (j < cnt)
+      for (int i = j >= 2 ? j - 2 : 0; i < j; ++i)
+        mbar_wait(landed + (i & 1), (i >> 1) & 1, nullptr, 0);
     return;
   }
 
   // -------------------------------------------------------------- consumers
-  float *const F = (float *)(ws_smem + (Lay::kDirect ? Lay::kS : Lay::kF));
-  float *const V = (float *)(ws_smem + Lay::kV);
-  const int x = t & 7, y = (t >> 3) & 7, z = t >> 6;
-  const CellMask cm{x > 0, x < 7, y > 0, y < 7, z > 0, z < 7};
-  const int eo = e_index(x, y, z);
   HaloRegs h;
-  for (int j = 0; j < cnt; ++j) {
-    const int r = j & (kWsRing - 1);
-    const bool ok = mbar_wait(landed, j & 1, fault, kWsFaultConsumerWait);
-    if (!consumer_sync_and(ok)) break;  // also: every consumer is done pulling item j-1
+  float hv[3] = {0.0f, 0.0f, 0.0f};
+  auto load = [&](int p) {
+    const int r = p & (kWsRing - 1);
     const LevelDev &L = BATCHED ? Ls[r] : L0;
-    const int *nbase = nbb[r];
+    ws_halo_load((const float *)L.f_in, dstride, wide, grow[r], nbb[r], t, tabs, h);
+    if (WALE) ws_vel_load(L, blk[r], nbb[r], t, hv);
+  };
+  for (int j = 0; j < cnt; ++j) {
+    const int r = j & (kWsRing - 1), bi = j & 1;
+    unsigned char *const buf = ws_smem + bi * kWsBuf;
+    float *const S = (float *)(buf + kWsS);
+    float *const V = (float *)(buf + kWsV);
+    const bool ok = mbar_wait(landed + bi, (j >> 1) & 1, fault, kWsFaultConsumerWait);
+    const LevelDev &L = BATCHED ? Ls[r] : L0;
+    const int *const nb = nbb[r];
     const int b = blk[r];
-    if (j == 0) ws_halo_load<ST, WALE>(L, b, nbase, t, tabs, h);
-    if constexpr (!Lay::kDirect) {
-      // spread the landed block into the pre-streamed stage
-#pragma unroll
-      for (int k = 0; k < 27; ++k)
-        if (pull_inside(cm, k))
-          F[k * BCELLS + t + cx_of(k) + 8 * cy_of(k) + 64 * cz_of(k)] =
-              land_value(ld, k, t, L.inv_scale, ST{});
-    }
-    // this thread's out-of-block values into the slots of the cells that pull them
-    const bool ghost = ghost_row_of(L, b) != nullptr;
-#pragma unroll
-    for (int m = 0; m < kWsHaloPerConsumer; ++m) {
-      const int i = t + BCELLS * m;
-      if (i >= kHaloEntries) continue;
-      const uint32_t e = tabs[i];
-      const int k = e & 31, dir = (e >> 5) & 31, d = e >> 19;
-      const float v = (nbase[dir] >= 0 || ghost)
-                          ? h.f[m]
-                          : pull_boundary<ST>(L, k, b, d & 7, (d >> 3) & 7, d >> 6);
-      if constexpr (Lay::kDirect) F[tabs[kWsSlotOffset + i]] = v;
-      else F[k * BCELLS + d] = v;
-    }
-    if (WALE) {
-      const float *lv = (const float *)(ld + Lay::kLdV);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) V[c * EPL + eo] = lv[c * BCELLS + t];
-      if (t < kWsVelEntries) {
-        const uint32_t e = tabs[kHaloEntries + t];
-        const int dir = e & 31, oc = (int)(e >> 5);
-        const int dx = dir % 3 - 1, dy = (dir / 3) % 3 - 1, dz = dir / 9 - 1;
-        const int slot = e_index(oc & 7, (oc >> 3) & 7, oc >> 6) + dx + 10 * dy + 100 * dz;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) V[c * EPL + slot] = h.v[c];
-      }
-    }
     CellAux aux;
-    aux.wall_dist = ((const float *)(ld + Lay::kLdWD))[t];
-    const float spg = ((const float *)(ld + Lay::kLdSP))[t];
-    const bool obs = ld[Lay::kLdOB + t] != 0;
-    if constexpr (!Lay::kDirect) {
-      // the landing buffer is read: the producer may fill it with item j+1
-      if (j + 1 < cnt) {
-        __syncwarp();
-        if ((t & 31) == 0) mbar_arrive(lfree);
+    float spg = 0.0f;
+    bool obs = false;
+    if (ok) {
+      if (j == 0) load(0);
+      ws_halo_store(S, nb, t, tabs, h, absent[r] && !grow[r], [&](int k, int x, int y, int z) {
+        return pull_boundary<StoreF32>(L, k, b, x, y, z);
+      });
+      if (WALE && t < 256) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) V[c * kWsVPlane + BCELLS + t] = hv[c];
       }
+      aux.wall_dist = ((const float *)(buf + kWsWD))[t];
+      spg = ((const float *)(buf + kWsSP))[t];
+      obs = buf[kWsOB + t] != 0;
     }
-    consumer_sync();  // the stage holds item j
+    if (!consumer_sync_and(ok)) break;  // the stage holds item j
+    aux.nu_wale = WALE ? ws_wale(V, t, L.sp.c_wale) : 0.0f;
     float A[27];
-    if constexpr (Lay::kDirect) {
 #pragma unroll
-      for (int k = 0; k < 27; ++k) A[k] = F[k * kSPlane + kSPad + t - cx_of(k)];
-      // the stage (also the landing buffer) is read: order these shared-memory
-      // accesses before the bulk copies of item j+1, then release it
-      if (j + 1 < cnt) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if ((t & 31) == 0) mbar_arrive(lfree);
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < 27; ++k) A[k] = F[k * BCELLS + t];
-    }
+    for (int k = 0; k < 27; ++k) A[k] = S[k * kSPlane + kSPad + t - cx_of(k)];
+    // the buffer is read: order these shared-memory accesses before the bulk
+    // copies of item j+2, then release it
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if ((t & 31) == 0) mbar_arrive(lfree + bi);
     // item j+1's out-of-block values, in flight while item j collides
-    if (j + 1 < cnt) {
-      const int r1 = (j + 1) & (kWsRing - 1);
-      ws_halo_load<ST, WALE>(BATCHED ? Ls[r1] : L0, blk[r1], nbb[r1], t, tabs, h);
-    }
-    if (WALE) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        aux.wale.e[c] = V[c * EPL + eo + 1];
-        aux.wale.w[c] = V[c * EPL + eo - 1];
-        aux.wale.n[c] = V[c * EPL + eo + 10];
-        aux.wale.s[c] = V[c * EPL + eo - 10];
-        aux.wale.t[c] = V[c * EPL + eo + 100];
-        aux.wale.b[c] = V[c * EPL + eo - 100];
-      }
-    }
-    collide_cell<OP, ST, WALE>(L, nbase, A, b, t, obs, spg, &aux);
+    if (j + 1 < cnt) load(j + 1);
+    collide_cell<OP, StoreF32, WALE>(L, nb, A, b, t, obs, spg, &aux);
   }
 }
 
