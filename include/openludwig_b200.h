@@ -151,7 +151,7 @@ OL_API int ol_stream_collide(const ol_level_view *lv, const ol_parent_view *pv,
  * launch shape).  OL_SC_KERNEL_BLOCK: one CTA per 8^3 block, synchronous
  * staging.  OL_SC_KERNEL_WS: one persistent CTA per SM whose producer warp
  * bulk-copies the next block while its consumer warps collide the current
- * one (cumulant operator, levels whose absent-neighbour values are ghost rows
+ * one (FP32, levels whose absent-neighbour values are ghost rows
  * or level-1 domain boundaries; other launches keep the per-block kernel).
  * The same choice applies to ol_thermal (FP32 thermal populations, two
  * blocks in flight per SM).

@@ -563,7 +563,7 @@ static int shape_for(const ol_ctx *c, const Launch &l) {
 
 template <int OP, class ST, bool WALE, bool DDF>
 static void launch_variant(ol_ctx *c, const Launch &l) {
-  if constexpr (OP == OL_OP_CUMULANT && !DDF && std::is_same<ST, StoreF32>::value) {
+  if constexpr (!DDF && std::is_same<ST, StoreF32>::value) {
     // FP32 storage only (FP16-shifted populations measured slower this way:
     // the consumers had to decode every landed value)
     const int choice = stream_collide_kernel_choice();
@@ -880,6 +880,8 @@ static int prepare_attributes() {
   prepare_attributes_st<StoreF16S>();
   cudaFuncSetAttribute(k_sc_ws<0, false, true>, (cudaFuncAttribute)a, kWsBytes);
   cudaFuncSetAttribute(k_sc_ws<0, true, true>, (cudaFuncAttribute)a, kWsBytes);
+  cudaFuncSetAttribute(k_sc_ws<1, false, true>, (cudaFuncAttribute)a, kWsBytes);
+  cudaFuncSetAttribute(k_sc_ws<1, true, true>, (cudaFuncAttribute)a, kWsBytes);
   if (!fault_word_device() || !ws_loader_device())
     return set_error(OL_ERR_CUDA, "warp-specialised kernel tables: allocation failed");
   const cudaError_t e = cudaGetLastError();

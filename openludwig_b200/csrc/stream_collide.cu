@@ -219,11 +219,10 @@ int ws_grid(int64_t n_items, int n_sm) {
 }
 
 // One CTA per block: neighbour offsets, then the staged pull windows, then
-// the cell update.  Cumulant fits 64 registers (2 CTAs of 512 threads per
-// SM, 2 x 105 KB of staging); regularized BGK keeps 27 equilibria in flight
-// and gets 128.
+// the cell update.  Both operators fit 64 registers (2 CTAs of 512 threads per
+// SM, 2 x 105 KB of staging).
 template <int OP, class ST, bool WALE>
-__global__ void __launch_bounds__(512, OP == OL_OP_CUMULANT ? 2 : 1)
+__global__ void __launch_bounds__(512, 2)
     k_stream_collide(const __grid_constant__ LevelDev L) {
   __shared__ int nbbase[27];
   extern __shared__ float E[];
@@ -296,13 +295,12 @@ static int device_sm_count() {
   return n_sm[dev];
 }
 
-// Whether the warp-specialised kernel serves this level: cumulant operator;
+// Whether the warp-specialised kernel serves this level:
 // every absent-neighbour value either precomputed in ghost rows or a
 // level-1 domain-boundary value its loader evaluates; the arrays it moves
 // with bulk copies 16-byte aligned.
 static bool ws_applies(const LevelDev &L) {
   auto a16 = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
-  if (L.sp.op != OL_OP_CUMULANT) return false;
   if (!L.sp.is_level_1 && !L.ghost) return false;
   if (!a16(L.f_in) || !a16(L.obstacle) || !a16(L.sponge)) return false;
   if (L.sp.c_wale != 0.0f && !a16(L.vel_in)) return false;
@@ -335,8 +333,13 @@ static void launch_sc(const LevelDev &L, cudaStream_t s) {
                   (g_sc_kernel == OL_SC_KERNEL_WS ||
                    (g_sc_kernel == OL_SC_KERNEL_AUTO && L.n_blocks >= 2 * n_sm));
   if (ws && ws_applies(L)) {
-    if (wale) launch_ws<OL_OP_CUMULANT, true>(L, n_sm, s);
-    else launch_ws<OL_OP_CUMULANT, false>(L, n_sm, s);
+    if (L.sp.op == OL_OP_CUMULANT) {
+      if (wale) launch_ws<OL_OP_CUMULANT, true>(L, n_sm, s);
+      else launch_ws<OL_OP_CUMULANT, false>(L, n_sm, s);
+    } else {
+      if (wale) launch_ws<OL_OP_REGULARIZED_BGK, true>(L, n_sm, s);
+      else launch_ws<OL_OP_REGULARIZED_BGK, false>(L, n_sm, s);
+    }
     return;
   }
   if (L.sp.op == OL_OP_CUMULANT) {

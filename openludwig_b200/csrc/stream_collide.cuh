@@ -548,6 +548,61 @@ __device__ __forceinline__ void collide_cumulant(float (&A)[27], float ux, float
   for (int i = 0; i < 9; ++i) chim_bwd(A[3 * i], A[3 * i + 1], A[3 * i + 2], ux);
 }
 
+// ---------------------------------------------------------------------------
+// Regularized BGK (kernel_regularized_bgk.jl:270-300).  A holds raw x-moments
+// on entry and populations on exit.  The second moments of the
+// non-equilibrium are those of the populations minus the equilibrium's, which
+// are polynomials in u on this lattice (c_a in {-1, 0, 1}): rho (1/3 + u_a^2)
+// and rho u_a u_b for O(u^2); the O(u^4) terms add -3/4 rho u_a^4 on the
+// diagonal and nothing off it.  So the 27 equilibria are needed once instead
+// of twice, and each is the even part of its direction pair plus or minus the
+// odd one: 13 pairs instead of 54 evaluations, and the populations are dead
+// before the first is formed (the kernel fits the warp-specialised form's 96
+// registers).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void bgk_regularized(float (&A)[27], float rho, float ux, float uy,
+                                                float uz, float om1, int comp) {
+  // sum_k f_k c_a c_b from the x-moments: rows i = (c_y + 1) + 3 (c_z + 1)
+  const float Sxx = (A[2] + A[5] + A[8]) + (A[11] + A[14] + A[17]) + (A[20] + A[23] + A[26]);
+  const float Syy = (A[0] + A[6]) + (A[9] + A[15]) + (A[18] + A[24]);
+  const float Szz = (A[0] + A[3] + A[6]) + (A[18] + A[21] + A[24]);
+  const float Sxy = (A[7] - A[1]) + (A[16] - A[10]) + (A[25] - A[19]);
+  const float Szx = (A[19] + A[22] + A[25]) - (A[1] + A[4] + A[7]);
+  const float Syz = (A[0] - A[6]) + (A[24] - A[18]);
+  const float xx = ux * ux, yy = uy * uy, zz = uz * uz, usq = xx + yy + zz;
+  const float a4 = comp ? -0.75f : 0.0f;
+  const float r3 = third_of(rho);
+  const float g = 4.5f * om1, g2 = 9.0f * om1;
+  const float qxx = g * (Sxx - fmaf(rho, fmaf(a4 * xx, xx, xx), r3));
+  const float qyy = g * (Syy - fmaf(rho, fmaf(a4 * yy, yy, yy), r3));
+  const float qzz = g * (Szz - fmaf(rho, fmaf(a4 * zz, zz, zz), r3));
+  const float qxy = g2 * (Sxy - rho * ux * uy);
+  const float qyz = g2 * (Syz - rho * uy * uz);
+  const float qzx = g2 * (Szx - rho * uz * ux);
+  const float tr = third_of(qxx + qyy + qzz);
+  // even part w (base + cu^2 (e2 + e4 cu^2) + q), odd part w cu (o1 + o3 cu^2)
+  const float base = rho * (comp ? fmaf(usq, fmaf(1.125f, usq, -1.5f), 1.0f)
+                                 : fmaf(-1.5f, usq, 1.0f)) - tr;
+  const float e2 = rho * (comp ? fmaf(-6.75f, usq, 4.5f) : 4.5f), e4 = comp ? 3.375f * rho : 0.0f;
+  const float o1 = rho * (comp ? fmaf(-4.5f, usq, 3.0f) : 3.0f), o3 = comp ? 4.5f * rho : 0.0f;
+  A[13] = w_of(13) * base;
+#pragma unroll
+  for (int k = 14; k < 27; ++k) {
+    const int cx = cx_of(k), cy = cy_of(k), cz = cz_of(k);
+    float cu = 0.0f, q = base;
+    if (cx) { cu = cx > 0 ? ux : -ux; q += qxx; }
+    if (cy) { cu = cy > 0 ? cu + uy : cu - uy; q += qyy; }
+    if (cz) { cu = cz > 0 ? cu + uz : cu - uz; q += qzz; }
+    if (cx * cy) q = cx * cy > 0 ? q + qxy : q - qxy;
+    if (cy * cz) q = cy * cz > 0 ? q + qyz : q - qyz;
+    if (cz * cx) q = cz * cx > 0 ? q + qzx : q - qzx;
+    const float c2 = cu * cu;
+    const float even = fmaf(c2, fmaf(e4, c2, e2), q), odd = cu * fmaf(o3, c2, o1);
+    A[k] = w_of(k) * (even + odd);
+    A[26 - k] = w_of(k) * (even - odd);
+  }
+}
+
 // Positivity limiter (kernel_cumulant.jl:564-599).
 __device__ __forceinline__ void positivity_limit(float (&A)[27], float rho, float ux, float uy,
                                               float uz, int comp) {
@@ -1262,25 +1317,14 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
     out.template f_all<true>(A);
     return;
   }
-  if constexpr (OP == OL_OP_CUMULANT) {
-    // A becomes the raw x-moments (m0, m1, m2) of each (y, z) triple
+  // A becomes the raw x-moments (m0, m1, m2) of each (y, z) triple
 #pragma unroll
-    for (int i = 0; i < 9; ++i) raw_moments(A[3 * i], A[3 * i + 1], A[3 * i + 2]);
-    const float s0 = A[0] + A[3] + A[6], s1 = A[9] + A[12] + A[15], s2 = A[18] + A[21] + A[24];
-    rho = s0 + s1 + s2;
-    jx = (A[1] + A[4] + A[7]) + (A[10] + A[13] + A[16]) + (A[19] + A[22] + A[25]);
-    jy = (A[6] - A[0]) + (A[15] - A[9]) + (A[24] - A[18]);
-    jz = s2 - s0;
-  } else {
-    rho = jx = jy = jz = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 27; ++k) {
-      rho += A[k];
-      if (cx_of(k) == 1) jx += A[k]; else if (cx_of(k) == -1) jx -= A[k];
-      if (cy_of(k) == 1) jy += A[k]; else if (cy_of(k) == -1) jy -= A[k];
-      if (cz_of(k) == 1) jz += A[k]; else if (cz_of(k) == -1) jz -= A[k];
-    }
-  }
+  for (int i = 0; i < 9; ++i) raw_moments(A[3 * i], A[3 * i + 1], A[3 * i + 2]);
+  const float s0 = A[0] + A[3] + A[6], s1 = A[9] + A[12] + A[15], s2 = A[18] + A[21] + A[24];
+  rho = s0 + s1 + s2;
+  jx = (A[1] + A[4] + A[7]) + (A[10] + A[13] + A[16]) + (A[19] + A[22] + A[25]);
+  jy = (A[6] - A[0]) + (A[15] - A[9]) + (A[24] - A[18]);
+  jz = s2 - s0;
   // device watchdog (native path): report, never trap
   if (L.status) watchdog(L.status, rho);
   rho = fminf(fmaxf(rho, 0.01f), 3e38f);
@@ -1299,7 +1343,7 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
         for (int j = 0; j < 3; ++j)
           ft[j] = feq_auto(1.0f, sp.u_inlet, 0.0f, 0.0f, w_of(3 * i + j), (float)cx_of(3 * i + j),
                            (float)cy_of(3 * i + j), (float)cz_of(3 * i + j), sp.compressible_corr);
-        if (OP == OL_OP_CUMULANT) raw_moments(ft[0], ft[1], ft[2]);
+        raw_moments(ft[0], ft[1], ft[2]);
 #pragma unroll
         for (int j = 0; j < 3; ++j) A[3 * i + j] = A[3 * i + j] * (1.0f - spg) + ft[j] * spg;
       }
@@ -1351,27 +1395,7 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
     // an undefined `cu`).
     const float tau_turb = sp.tau_molecular + nu_eddy * 3.0f;
     omega = recip_nr(fminf(fmaxf(tau_turb, 0.500001f), 3e38f));
-    float Pxx = 0.f, Pyy = 0.f, Pzz = 0.f, Pxy = 0.f, Pyz = 0.f, Pzx = 0.f;
-#pragma unroll
-    for (int k = 0; k < 27; ++k) {
-      const float cxf = (float)cx_of(k), cyf = (float)cy_of(k), czf = (float)cz_of(k);
-      const float fn = A[k] - feq_auto(rho, uxe, uye, uze, w_of(k), cxf, cyf, czf,
-                                       sp.compressible_corr);
-      Pxx += fn * cxf * cxf; Pyy += fn * cyf * cyf; Pzz += fn * czf * czf;
-      Pxy += fn * cxf * cyf; Pyz += fn * cyf * czf; Pzx += fn * czf * cxf;
-    }
-    const float cs2p = 1.0f / 3.0f;
-#pragma unroll
-    for (int k = 0; k < 27; ++k) {
-      const float cxf = (float)cx_of(k), cyf = (float)cy_of(k), czf = (float)cz_of(k);
-      const float w = w_of(k);
-      const float fe = feq_auto(rho, uxe, uye, uze, w, cxf, cyf, czf, sp.compressible_corr);
-      const float fr = w * 4.5f *
-                       (Pxx * (cxf * cxf - cs2p) + Pyy * (cyf * cyf - cs2p) +
-                        Pzz * (czf * czf - cs2p) +
-                        2.0f * (Pxy * cxf * cyf + Pyz * cyf * czf + Pzx * czf * cxf));
-      A[k] = fe + (1.0f - omega) * fr;
-    }
+    bgk_regularized(A, rho, uxe, uye, uze, 1.0f - omega, sp.compressible_corr);
   }
   if (forced) {
     const float g = 1.0f - 0.5f * omega;

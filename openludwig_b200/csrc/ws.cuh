@@ -28,16 +28,16 @@
 // then the 6 x 64 values beyond the faces (a face without a neighbour repeats
 // the cell beside it, the zero-gradient fallback of the WALE gradients).
 //
-// Why this split (measured on B200, cube_3lvl, us per coarse step of this
-// kernel): an SM has to keep ~60-90 KB in flight to draw its share of HBM
-// bandwidth, which bulk copies do and loader warps do not (see the variants in
-// the design notes).  With one stage buffer the next landing could only start
-// after the pulls and end before the next item, so the consumers waited for
-// it: 905 us; with two buffers, z layers by bulk copy and one barrier 766 us
-// (sphere_ddf: 291 -> 260 us, the thermal kernel built the same way 245 -> 222)  Of the 3176 out-of-block
-// sources 968 lie in the z neighbours' contiguous layers and come by bulk copy;
-// the consumers carry the other 2208 (5 registers a thread instead of 7), each
-// found by one 8-byte table entry whose plane offset is formed once per launch.
+// Why this split (measured on B200): an SM has to keep ~60-90 KB in flight to
+// draw its share of HBM bandwidth, which bulk copies do and loader warps do
+// not.  With one stage buffer the next landing could only start after the
+// pulls and had to end before the next item, so the consumers waited for it:
+// 905 us per coarse step of cube_3lvl; with two buffers, z layers by bulk copy
+// and one barrier 766 us (sphere_ddf 291 -> 260 us, the thermal kernel built
+// the same way 245 -> 222 us).  Of the 3176 out-of-block sources 968 lie in the
+// z neighbours' contiguous layers and come by bulk copy; the consumers carry
+// the other 2208 (5 registers a thread instead of 7), each found by one 8-byte
+// table entry whose plane offset is formed once per launch.
 //
 // Hand-over uses mbarriers ("landed": bulk bytes plus the producer's arrival;
 // "free": one arrival per consumer warp, both per buffer) and one named barrier
@@ -342,6 +342,9 @@ __device__ __forceinline__ float ws_wale(const float *V, int t, float c_wale) {
   return wale_from(w, c_wale);
 }
 
+// Both operators: the regularized-BGK update needs fewer registers than the
+// cumulant one; its levels took 335 us per coarse step of a 2-level sphere of
+// 32 cells with one CTA per block and 202 us here.
 template <int OP, bool WALE, bool BATCHED>
 __global__ void __launch_bounds__(kWsThreads, 1)
     k_sc_ws(const __grid_constant__ LevelDev L0, const LevelDev *__restrict__ descs,
