@@ -604,6 +604,37 @@ typedef struct ol_restrict_view {
 OL_API int ol_restrict(const ol_restrict_view *v, void *stream);
 
 /* ------------------------------------------------------------------------
+ * A batch of coarse time steps in one call (execute_timestep_batch!,
+ * solver_control.jl:199-218): steps t_start .. t_start + n_steps - 1 of the
+ * 2:1 recursion, each level sub-step through the entry points above, on
+ * `stream`.  The buffers stay the caller's.
+ * ------------------------------------------------------------------------ */
+typedef struct ol_march_level {
+  /* f_in / vel_in are the buffers read on the level's even sub-steps and
+   * f_out / vel_out those it writes then (exchanged on odd ones); ghost and
+   * ghost_next the two ghost scratches (either NULL: no pairing / no pass);
+   * ghost_blocks the visit list; f_post and ghost_mode are not read. */
+  ol_level_view view;
+  const int32_t *edge_blocks;       /* visit list of a pair's second sub-step   */
+  int32_t n_edge_blocks;
+  float *rho_old;                   /* [512*nB], levels with children           */
+  const int32_t *block_ptr;         /* as ol_parent_view                        */
+  int32_t dim_x, dim_y, dim_z;
+  float tau, tau_g;
+  const ol_bouzidi_link *links;     /* cut links (ol_bouzidi_build_links)       */
+  int32_t n_links;
+  float *link_scratch;              /* [n_links]                                */
+  float *g, *g_temp, *temperature, *temperature_old; /* thermal DDF, or NULL    */
+  float *ghost_g, *ghost_g2;        /* ghost scratches of g, or NULL            */
+} ol_march_level;
+/* sp, tp: the scalars all levels share (tau*, level, sizes, weight, seed and
+ * store_post_collision are set per sub-step); tp NULL = no thermal DDF.
+ * nx, ny, nz: level 1's size in cells.  restriction != 0 adds ol_restrict. */
+OL_API int ol_march(const ol_march_level *levels, int32_t n_levels, const ol_step_params *sp,
+                    const ol_thermal_params *tp, int32_t restriction, int32_t nx, int32_t ny,
+                    int32_t nz, int64_t t_start, int32_t n_steps, void *stream);
+
+/* ------------------------------------------------------------------------
  * Domain preprocessing on the device (the host build is the reference's
  * CPU path; these give the same bits).  All pointers are device memory:
  *   coords   [n_blocks][3] 1-based block coordinates (x, y, z) of the level

@@ -81,6 +81,14 @@ class RestrictView(C.Structure):
                 ("tau_coarse", f32), ("compressible", i32)]
 
 
+class MarchLevel(C.Structure):
+    _fields_ = [("view", LevelView), ("edge_blocks", vp), ("n_edge_blocks", i32), ("rho_old", vp),
+                ("block_ptr", vp), ("dim_x", i32), ("dim_y", i32), ("dim_z", i32), ("tau", f32),
+                ("tau_g", f32), ("links", vp), ("n_links", i32), ("link_scratch", vp), ("g", vp),
+                ("g_temp", vp), ("temperature", vp), ("temperature_old", vp), ("ghost_g", vp),
+                ("ghost_g2", vp)]
+
+
 class FeMapView(C.Structure):
     _fields_ = [("node_xyz", vp), ("tri_xyz", vp), ("tri_force", vp), ("node_begin", vp),
                 ("tri_begin", vp), ("n_nodes", i32), ("n_tris", i32), ("n_objects", i32),
@@ -180,6 +188,8 @@ _SIGS = {
     "ol_bouzidi_apply_links": (C.c_int, [vp, vp, i32, i32, vp, vp]),
     "ol_thermal": (C.c_int, [C.POINTER(ThermalView), C.POINTER(ThermalParams), vp]),
     "ol_restrict": (C.c_int, [C.POINTER(RestrictView), vp]),
+    "ol_march": (C.c_int, [C.POINTER(MarchLevel), i32, C.POINTER(StepParams),
+                           C.POINTER(ThermalParams), i32, i32, i32, i32, C.c_int64, i32, vp]),
     "ol_voxelize": (C.c_int, [vp, i32, vp, i32, vp, vp, C.c_double, C.POINTER(C.c_double), vp,
                               vp]),
     "ol_bouzidi_qmap": (C.c_int, [vp, i32, vp, i32, vp, vp, C.c_double, C.POINTER(C.c_double),

@@ -299,6 +299,16 @@ def _ghost_views(view, lv: DeviceLevel, ghost, ghost2, mode: int) -> None:
         view.ghost_blocks, view.n_ghost_blocks = _ptr(lst), int(lst.numel()) - 1
 
 
+def build_ghost_lists(lv: DeviceLevel, dims) -> None:
+    """The ghost pass's visit lists: static, computed on first use."""
+    if lv.ghost is not None and lv.ghost_list is None:
+        # one trailing entry keeps an empty list's pointer non-null (a null
+        # list means "every block"); the view passes the true length
+        gl, el = ghost_block_lists(lv.host, dims)
+        lv.ghost_list = torch.from_numpy(np.append(gl, -1).astype(np.int32)).to(lv.f.device)
+        lv.edge_list = torch.from_numpy(np.append(el, -1).astype(np.int32)).to(lv.f.device)
+
+
 def perform_timestep(s: StepSettings, lv: DeviceLevel, parent: ParentRef | None, f_out, f_in,
                      vel_out, vel_in, u: float, t_sub: int, tw: float, domain_dims,
                      g_out=None, g_in=None, ghost_mode: int = 0) -> None:
@@ -312,12 +322,7 @@ def perform_timestep(s: StepSettings, lv: DeviceLevel, parent: ParentRef | None,
     scale = 1 << (lv.host.level_id - 1)
     dims = (domain_dims[0] * scale, domain_dims[1] * scale, domain_dims[2] * scale)
     ref_post = lv.f_post is not None
-    if lv.ghost is not None and lv.ghost_list is None:   # static: computed on first use
-        # one trailing entry keeps an empty list's pointer non-null (a null
-        # list means "every block"); the view passes the true length
-        gl, el = ghost_block_lists(lv.host, dims)
-        lv.ghost_list = torch.from_numpy(np.append(gl, -1).astype(np.int32)).to(lv.f.device)
-        lv.edge_list = torch.from_numpy(np.append(el, -1).astype(np.int32)).to(lv.f.device)
+    build_ghost_lists(lv, dims)
     sp = step_params(s, lv, parent.lv.tau if parent else 0.5, is_l1, dims, u, t_sub, tw,
                      lv.has_bouzidi and ref_post)
     view = N.LevelView(f_out=_ptr(f_out), f_in=_ptr(f_in), f_post=_ptr(lv.f_post),
@@ -442,11 +447,69 @@ def restrict_level(child: DeviceLevel, parent: ParentRef, s: StepSettings) -> No
     N.call("ol_restrict", C.byref(v), _stream())
 
 
+def _march_level(s: StepSettings, lv: DeviceLevel, i: int, domain_dims) -> N.MarchLevel:
+    """A level's buffers as ol_march reads them (pointers taken per batch)."""
+    scale = 1 << i
+    m = N.MarchLevel()
+    m.view = N.LevelView(f_out=_ptr(lv.f_temp), f_in=_ptr(lv.f), rho=_ptr(lv.rho),
+                         vel_out=_ptr(lv.vel_temp), vel_in=_ptr(lv.vel),
+                         obstacle=_ptr(lv.obstacle), sponge=_ptr(lv.sponge),
+                         wall_dist=_ptr(lv.wall_dist), neighbor_table=_ptr(lv.neighbor_table),
+                         map_x=_ptr(lv.map_x), map_y=_ptr(lv.map_y), map_z=_ptr(lv.map_z),
+                         ghost=_ptr(lv.ghost), ghost_next=_ptr(lv.ghost2), n_blocks=lv.n_blocks)
+    if lv.n_blocks:
+        build_ghost_lists(lv, tuple(d * scale for d in domain_dims))
+    if lv.ghost_list is not None:
+        m.view.ghost_blocks = _ptr(lv.ghost_list)
+        m.view.n_ghost_blocks = int(lv.ghost_list.numel()) - 1
+        m.edge_blocks, m.n_edge_blocks = _ptr(lv.edge_list), int(lv.edge_list.numel()) - 1
+    m.rho_old, m.block_ptr = _ptr(lv.rho_old), _ptr(lv.block_ptr)
+    m.dim_x, m.dim_y, m.dim_z = lv.host.grid_dim
+    m.tau, m.tau_g = lv.tau, lv.host.tau_g
+    if lv.has_bouzidi and lv.n_blocks:
+        if lv.bz_links is None:
+            build_bouzidi_links(lv, s.q_min)
+        m.links, m.n_links = _ptr(lv.bz_links), lv.bz_n_links
+        m.link_scratch = _ptr(lv.bouzidi_scratch)
+    if s.ddf:
+        m.g, m.g_temp = _ptr(lv.g), _ptr(lv.g_temp)
+        m.temperature, m.temperature_old = _ptr(lv.temperature), _ptr(lv.temperature_old)
+        m.ghost_g, m.ghost_g2 = _ptr(lv.ghost_g), _ptr(lv.ghost_g2)
+    return m
+
+
 def execute_timestep_batch(levels, s: StepSettings, t_start: int, batch: int, u: float,
                            domain_dims) -> None:
-    """solver_control.jl:199-218."""
-    for off in range(batch):
-        recursive_step(levels, s, 0, t_start + off, None, 0.0, u, domain_dims)
+    """solver_control.jl:199-218, as one library call (ol_march).  Levels that
+    keep the reference's post-collision copy, or whose scale is not their
+    place in the list, step through recursive_step."""
+    if batch <= 0 or not levels:
+        return
+    if any(lv.f_post is not None or lv.host.level_id != i + 1
+           or (s.ddf and (lv.g is None or lv.temperature is None))
+           for i, lv in enumerate(levels)):
+        for off in range(batch):
+            recursive_step(levels, s, 0, t_start + off, None, 0.0, u, domain_dims)
+        return
+    lvs = (N.MarchLevel * len(levels))(*[_march_level(s, lv, i, domain_dims)
+                                         for i, lv in enumerate(levels)])
+    sp = step_params(s, levels[0], 0.5, True, domain_dims, u, 0, 0.0, False)
+    tp = None
+    if s.ddf:
+        tp = C.byref(N.ThermalParams(u_inlet=u, T_inlet=s.t_inlet, T_wall=s.t_wall,
+                                     is_symmetric=s.is_symmetric,
+                                     wall_bc_adiabatic=s.wall_bc_adiabatic,
+                                     use_temporal_interp=s.use_temporal_interp,
+                                     sponge_blend_distributions=s.sponge_blend))
+    N.call("ol_march", lvs, N.i32(len(levels)), C.byref(sp), tp, N.i32(int(s.restriction)),
+           *(N.i32(d) for d in domain_dims), C.c_int64(t_start), N.i32(batch), _stream())
+    if s.use_temporal_interp:
+        # the parent state the last step's children read, as recursive_step leaves it
+        for i, lv in enumerate(levels[:-1]):
+            even = i == 0 and (t_start + batch - 1) % 2 == 0
+            lv.f_old, lv.vel_old = (lv.f, lv.vel) if even else (lv.f_temp, lv.vel_temp)
+            if s.ddf:
+                lv.g_old = lv.g if even else lv.g_temp
 
 
 @dc.dataclass

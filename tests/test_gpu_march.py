@@ -1,0 +1,63 @@
+"""A batch of coarse steps in one library call (ol_march) against the same
+steps driven one level sub-step at a time (solver.recursive_step): the same
+entry points with the same arguments, so every buffer is bitwise equal."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from helpers import small_sphere_case
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():  # pragma: no cover - CPU container
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+from openludwig_b200 import _native as N  # noqa: E402
+from openludwig_b200 import solver as S  # noqa: E402
+
+DEV = torch.device("cuda:0")
+CASES = [
+    dict(name="one_level", levels=1),
+    dict(name="refined", levels=2, c_wale=np.float32(0.5), inlet_turbulence_intensity=0.02),
+    dict(name="no_temporal", levels=2, temporal_interpolation=False),
+    dict(name="restriction", levels=2, fine_to_coarse_restriction=True),
+    dict(name="thermal", levels=2, compressibility_correction=True, ddf_enabled=True,
+         u_target=np.float32(0.1), sponge_blend_distributions=True),
+]
+
+
+@pytest.mark.parametrize("first,steps", [(1, 1), (1, 3), (4, 2)])
+@pytest.mark.parametrize("case", CASES, ids=[c["name"] for c in CASES])
+def test_batch_equals_single_sub_steps(case, first, steps):
+    kw = {k: v for k, v in case.items() if k not in ("name", "levels")}
+    c, mesh, p, hosts = small_sphere_case(resolution=16 if case["levels"] > 1 else 8,
+                                          levels=case["levels"], **kw)
+    st = S.StepSettings.from_config(c, False)
+    dims, u = (p.nx_coarse, p.ny_coarse, p.nz_coarse), float(c.u_target)
+    runs = []
+    for batch in (False, True):
+        levels = [S.upload_level(h, DEV, ddf=c.ddf_enabled) for h in hosts]
+        if batch:
+            S.execute_timestep_batch(levels, st, first, steps, u, dims)
+        else:
+            for k in range(steps):
+                S.recursive_step(levels, st, 0, first + k, None, 0.0, u, dims)
+        torch.cuda.synchronize()
+        runs.append(levels)
+    names = ["f", "f_temp", "rho", "vel", "vel_temp"] + (["g", "g_temp", "temperature"]
+                                                          if c.ddf_enabled else [])
+    for i, (a, b) in enumerate(zip(*runs)):
+        for n in names:
+            assert torch.equal(getattr(a, n), getattr(b, n)), (i, n)
+        if i + 1 < len(hosts) and st.use_temporal_interp:
+            assert torch.equal(a.f_old, b.f_old) and torch.equal(a.rho_old, b.rho_old)
+
+
+def test_march_reports_bad_arguments():
+    lv = (N.MarchLevel * 1)()
+    with pytest.raises(N.OLError):
+        N.call("ol_march", lv, 0, C.byref(N.StepParams()), None, 0, 8, 8, 8, 1, 1, None)
+    with pytest.raises(N.OLError):  # thermal parameters without thermal buffers
+        N.call("ol_march", lv, 1, C.byref(N.StepParams()), C.byref(N.ThermalParams()), 0, 8, 8, 8,
+               1, 1, None)
