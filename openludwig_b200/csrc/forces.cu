@@ -227,65 +227,87 @@ __global__ void __launch_bounds__(kForceThreads)
   M.net_fz[i] = -pn * nz * A + snz * A;
 }
 
-// Fixed-order sum of nvals-wide partial rows: out[j] = sum_b partials[b*nvals + j].
-__global__ void k_sum_rows(const double *partials, int nrows, int nvals, double *out,
-                           int mode_minmax) {
-  __shared__ double sh[256];
-  for (int j = 0; j < nvals; ++j) {
-    const bool is_min = mode_minmax && j == 2;
-    const bool is_max = mode_minmax && (j == 3 || j == 4);
-    double s = is_min ? 1e300 : (is_max ? -1e300 : 0.0);
-    for (int r = threadIdx.x; r < nrows; r += blockDim.x) {
-      const double v = partials[(size_t)r * nvals + j];
-      s = is_min ? fmin(s, v) : (is_max ? fmax(s, v) : s + v);
-    }
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-      if (threadIdx.x < o) {
-        const double a = sh[threadIdx.x], b = sh[threadIdx.x + o];
-        sh[threadIdx.x] = is_min ? fmin(a, b) : (is_max ? fmax(a, b) : a + b);
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) out[j] = sh[0];
-    __syncthreads();
+// Fixed-order reduction of nvals-wide partial rows to out[nvals]: column j is
+// summed (mode_minmax: column 2 by minimum, 3 and 4 by maximum) by its own
+// kSumWarps warps, lane by lane over the rows, so the columns' loads overlap;
+// one thread block walking the columns one after another, each with a
+// barrier tree, took 14 us of the 44 us a diagnostics step's kernels took.
+constexpr int kSumWarps = 3, kSumMaxVals = 9;
+__device__ __forceinline__ double combine(int op, double a, double b) {
+  return op == 0 ? a + b : (op < 0 ? fmin(a, b) : fmax(a, b));
+}
+__global__ void __launch_bounds__(32 * kSumWarps * kSumMaxVals)
+    k_sum_rows(const double *__restrict__ partials, int nrows, int nvals, double *out,
+               int mode_minmax) {
+  __shared__ double sh[kSumMaxVals][kSumWarps];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int j = wid / kSumWarps, part = wid % kSumWarps;
+  const int op = !mode_minmax ? 0 : (j == 2 ? -1 : (j == 3 || j == 4 ? 1 : 0));
+  double s = op == 0 ? 0.0 : (op < 0 ? 1e300 : -1e300);
+#pragma unroll 4
+  for (int r = part * 32 + lane; r < nrows; r += 32 * kSumWarps)
+    s = combine(op, s, __ldg(partials + (size_t)r * nvals + j));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s = combine(op, s, __shfl_down_sync(0xffffffffu, s, o));
+  if (lane == 0) sh[j][part] = s;
+  __syncthreads();
+  if (threadIdx.x < nvals) {
+    const int c = threadIdx.x;
+    const int oc = !mode_minmax ? 0 : (c == 2 ? -1 : (c == 3 || c == 4 ? 1 : 0));
+    s = sh[c][0];
+    for (int w = 1; w < kSumWarps; ++w) s = combine(oc, s, sh[c][w]);
+    out[c] = s;
   }
+}
+static void sum_rows(const double *partials, int nrows, int nvals, double *out, int mode_minmax,
+                     cudaStream_t s) {
+  k_sum_rows<<<1, 32 * kSumWarps * nvals, 0, s>>>(partials, nrows, nvals, out, mode_minmax);
 }
 
 // Per-block FP64 flow statistics: {n_fluid, rho_sum, rho_min, rho_max,
-// v_max, kinetic_energy, mass_all}.
-__global__ void __launch_bounds__(512) k_flow_stats(const float *rho, const float *vel,
-                                                    const uint8_t *obs, int64_t block_offset,
-                                                    int64_t dstride, double *partials) {
-  const size_t ci = (size_t)(block_offset + blockIdx.x) * BCELLS + threadIdx.x;
-  const double r = rho[ci];
-  const double ux = vel[ci], uy = vel[ci + dstride], uz = vel[ci + 2 * dstride];
-  const double v2 = ux * ux + uy * uy + uz * uz;
-  const bool fluid = !obs[ci];
-  double v[7] = {fluid ? 1.0 : 0.0, fluid ? r : 0.0, fluid ? r : 1e300, fluid ? r : -1e300,
-                 fluid ? sqrt(v2) : 0.0, fluid ? 0.5 * r * v2 : 0.0, r};
-  __shared__ double red[16][7];
+// v_max, kinetic_energy, mass_all}.  Bound by the seven double-precision
+// shuffle reductions, so a thread first combines four cells (128 threads a
+// block instead of 512) and the root is taken once of the largest square.
+constexpr int kStatThreads = 128;
+__global__ void __launch_bounds__(kStatThreads)
+    k_flow_stats(const float *__restrict__ rho, const float *__restrict__ vel,
+                 const uint8_t *__restrict__ obs, int64_t block_offset, int64_t dstride,
+                 double *partials) {
+  const size_t c0 = (size_t)(block_offset + blockIdx.x) * BCELLS + threadIdx.x;
+  double v[7] = {0.0, 0.0, 1e300, -1e300, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int i = 0; i < BCELLS / kStatThreads; ++i) {
+    const size_t ci = c0 + i * kStatThreads;
+    const double r = rho[ci];
+    const double ux = vel[ci], uy = vel[ci + dstride], uz = vel[ci + 2 * dstride];
+    const double v2 = ux * ux + uy * uy + uz * uz;
+    v[6] += r;
+    if (!obs[ci]) {
+      v[0] += 1.0;
+      v[1] += r;
+      v[2] = fmin(v[2], r);
+      v[3] = fmax(v[3], r);
+      v[4] = fmax(v[4], v2);
+      v[5] += 0.5 * r * v2;
+    }
+  }
+  __shared__ double red[kStatThreads / 32][7];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
   for (int j = 0; j < 7; ++j) {
+    const int op = j == 2 ? -1 : (j == 3 || j == 4 ? 1 : 0);
     double x = v[j];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double y = __shfl_down_sync(0xffffffffu, x, o);
-      x = j == 2 ? fmin(x, y) : ((j == 3 || j == 4) ? fmax(x, y) : x + y);
-    }
+    for (int o = 16; o > 0; o >>= 1) x = combine(op, x, __shfl_down_sync(0xffffffffu, x, o));
     if (lane == 0) red[wid][j] = x;
   }
   __syncthreads();
   if (threadIdx.x < 7) {
     const int j = threadIdx.x;
+    const int op = j == 2 ? -1 : (j == 3 || j == 4 ? 1 : 0);
     double s = red[0][j];
-    for (int w = 1; w < 16; ++w) {
-      const double y = red[w][j];
-      s = j == 2 ? fmin(s, y) : ((j == 3 || j == 4) ? fmax(s, y) : s + y);
-    }
-    partials[(size_t)blockIdx.x * 7 + j] = s;
+    for (int w = 1; w < kStatThreads / 32; ++w) s = combine(op, s, red[w][j]);
+    partials[(size_t)blockIdx.x * 7 + j] = j == 4 ? sqrt(s) : s;
   }
 }
 
@@ -294,7 +316,7 @@ int launch_surface_forces(const ForceDev &D, double *dev_out9, cudaStream_t s) {
   const int grid = (nt + kForceThreads - 1) / kForceThreads;
   if (grid == 0) return 0;
   k_surface_forces<<<grid, kForceThreads, 0, s>>>(D);
-  k_sum_rows<<<1, 256, 0, s>>>(D.partials, grid, 9, dev_out9, 0);
+  sum_rows(D.partials, grid, 9, dev_out9, 0, s);
   return 0;
 }
 
@@ -302,8 +324,8 @@ int launch_flow_stats(const float *rho, const float *vel, const uint8_t *obs, in
                       int64_t block_offset, int64_t dstride, double *partials, double *dev_out7,
                       cudaStream_t s) {
   if (nb <= 0) return 0;
-  k_flow_stats<<<nb, 512, 0, s>>>(rho, vel, obs, block_offset, dstride, partials);
-  k_sum_rows<<<1, 256, 0, s>>>(partials, nb, 7, dev_out7, 1);
+  k_flow_stats<<<nb, kStatThreads, 0, s>>>(rho, vel, obs, block_offset, dstride, partials);
+  sum_rows(partials, nb, 7, dev_out7, 1, s);
   return 0;
 }
 

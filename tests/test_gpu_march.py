@@ -61,3 +61,23 @@ def test_march_reports_bad_arguments():
     with pytest.raises(N.OLError):  # thermal parameters without thermal buffers
         N.call("ol_march", lv, 1, C.byref(N.StepParams()), C.byref(N.ThermalParams()), 0, 8, 8, 8,
                1, 1, None)
+
+
+@pytest.mark.parametrize("blocks", [1, 3, 97, 300])
+def test_flow_statistics_of_any_block_count(blocks):
+    g = torch.Generator(device=DEV).manual_seed(blocks)
+    n = 512 * blocks
+    rho = 1 + 0.1 * torch.randn(n, generator=g, device=DEV)
+    vel = 0.1 * torch.randn(3 * n, generator=g, device=DEV)
+    obs = (torch.rand(n, generator=g, device=DEV) < 0.3).to(torch.uint8)
+    part = torch.empty(int(N.lib().ol_flow_stats_scratch_doubles(blocks)), dtype=torch.float64,
+                       device=DEV)
+    out = (C.c_double * 7)()
+    N.call("ol_flow_stats", rho.data_ptr(), vel.data_ptr(), obs.data_ptr(), N.i32(blocks),
+           part.data_ptr(), out, None)
+    r, v2 = rho.double(), vel.double().reshape(3, n).square().sum(0)
+    f = obs == 0
+    want = [f.sum(), r[f].sum(), r[f].min(), r[f].max(), v2[f].max().sqrt(),
+            (0.5 * r * v2)[f].sum(), r.sum()]
+    # FP64 sums of up to 1.5e5 terms in another order: n * 2^-53 at most
+    assert np.allclose(out[:], [float(w) for w in want], rtol=2e-11, atol=0)
