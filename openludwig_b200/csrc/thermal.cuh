@@ -78,17 +78,17 @@ __device__ __forceinline__ void ghost_moments(const ThermalDev &D, const ParentS
 }
 
 // g_eq(T, u) + (g - g_eq) * clamp(...) from the 8 corner values of g_k.
-__device__ __forceinline__ float finish_thermal(const ThermalDev &D, int k, const float (&v)[8],
+__device__ __forceinline__ GhostScale ghost_scale(const ThermalDev &D) {
+  return ghost_scale(D.tp.tau_g_parent, D.tp.tau_g, 0);
+}
+__device__ __forceinline__ float finish_thermal(const GhostScale &g, int k, const float (&v)[8],
                                                 float wx, float wy, float wz,
                                                 const float (&r)[4]) {
-  const ol_thermal_params &tp = D.tp;
   const float gi = trilerp(v, wx, wy, wz);
   const float ge = geq(r[0], r[1], r[2], r[3], w_of(k), (float)cx_of(k), (float)cy_of(k),
                        (float)cz_of(k));
   const float gneq = gi - ge;
-  const float tc = tp.tau_g_parent - 0.5f, tf = tp.tau_g - 0.5f;
-  const float sc = tc > 1e-6f ? fminf(fmaxf(tf / tc, 0.01f), 100.0f) : 1.0f;
-  return __fadd_rn(ge, __fmul_rn(gneq, sc));
+  return __fadd_rn(ge, __fmul_rn(gneq, g.sc));
 }
 
 template <class ST>
@@ -112,7 +112,7 @@ __device__ __forceinline__ float ghost_population(const ThermalDev &D, int k,
 #pragma unroll
   for (int s = 1; s < 8; ++s)
     if (P.ci[s] < 0) v[s] = v[0];
-  return finish_thermal(D, k, v, P.wx, P.wy, P.wz, r);
+  return finish_thermal(ghost_scale(D), k, v, P.wx, P.wy, P.wz, r);
 }
 
 // The ghost pass's view of the thermal level (stream_collide.cuh).
@@ -123,9 +123,10 @@ __device__ __forceinline__ const float *ghost_moment_plane(const ThermalDev &D, 
 __device__ __forceinline__ const void *ghost_parent(const ThermalDev &D, bool old) {
   return old ? D.pg_old : D.pg;
 }
-__device__ __forceinline__ float ghost_finish(const ThermalDev &D, int k, const float (&v)[8],
-                                              float wx, float wy, float wz, const float (&r)[4]) {
-  return finish_thermal(D, k, v, wx, wy, wz, r);
+__device__ __forceinline__ float ghost_finish(const ThermalDev &, const GhostScale &g, int k,
+                                              const float (&v)[8], float wx, float wy, float wz,
+                                              const float (&r)[4]) {
+  return finish_thermal(g, k, v, wx, wy, wz, r);
 }
 
 template <class ST>
@@ -192,7 +193,10 @@ __device__ __forceinline__ void thermal_cell(const ThermalDev &D, const int *nbb
   const int x = t & 7, y = (t >> 3) & 7, z = t >> 6;
   const ol_thermal_params &tp = D.tp;
   const size_t own = (size_t)nbbase[13] + t;
+  // the descriptor may lie in shared memory: fields the stores need, read once
   T *__restrict__ gout = (T *)D.g_out;
+  const int64_t dstride = D.dstride;
+  const float scale = D.scale;
   float ux = D.vel[own], uy = D.vel[own + D.dstride], uz = D.vel[own + 2 * D.dstride];
   const int eb = e_index(x, y, z);
   float G[27];
@@ -215,8 +219,8 @@ __device__ __forceinline__ void thermal_cell(const ThermalDev &D, const int *nbb
                              (float)cy_of(k), (float)cz_of(k));
         v = 2.0f * gw - gopp;
       }
-      ST::store(gout, own + (size_t)k * D.dstride, k, D.scale, v);
-      if (gpost) gpost[own + (size_t)k * D.dstride] = v;
+      ST::store(gout, own + (size_t)k * dstride, k, scale, v);
+      if (gpost) gpost[own + (size_t)k * dstride] = v;
     }
     D.T_out[own] = tp.wall_bc_adiabatic == 1 ? Tsum : tp.T_wall;
     return;
@@ -243,8 +247,8 @@ __device__ __forceinline__ void thermal_cell(const ThermalDev &D, const int *nbb
     }
     const float ge = geq(Tl, ux, uy, uz, w, cxf, cyf, czf);
     const float gc = gs - og * (gs - ge);
-    ST::store(gout, own + (size_t)k * D.dstride, k, D.scale, gc);
-    if (gpost) gpost[own + (size_t)k * D.dstride] = gc;
+    ST::store(gout, own + (size_t)k * dstride, k, scale, gc);
+    if (gpost) gpost[own + (size_t)k * dstride] = gc;
   }
 }
 
