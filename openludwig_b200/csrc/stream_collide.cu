@@ -268,16 +268,16 @@ static void launch_one(const LevelDev &L0, cudaStream_t s) {
 
 // Warp-specialised persistent kernel over the level's blocks: one CTA per
 // SM (or per block when the level is smaller).
-template <int OP, bool WALE>
+template <int OP, bool WALE, bool LOW = false>
 static void launch_ws(const LevelDev &L, int n_sm, cudaStream_t s) {
   static bool done = false;
   if (!done) {
-    cudaFuncSetAttribute(k_sc_ws<OP, WALE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_sc_ws<OP, WALE, false, LOW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          kWsBytes);
     done = true;
   }
   const int grid = ws_grid(L.n_blocks, n_sm);
-  launch_pdl(k_sc_ws<OP, WALE, false>, grid, kWsThreads, kWsBytes, s, L,
+  launch_pdl(k_sc_ws<OP, WALE, false, LOW>, grid, kWsThreads, kWsBytes, s, L,
              (const LevelDev *)nullptr, (const WorkItem *)nullptr, 0, ws_loader_device(),
              fault_word_device());
 }
@@ -333,7 +333,10 @@ static void launch_sc(const LevelDev &L, cudaStream_t s) {
                   (g_sc_kernel == OL_SC_KERNEL_WS ||
                    (g_sc_kernel == OL_SC_KERNEL_AUTO && L.n_blocks >= 2 * n_sm));
   if (ws && ws_applies(L)) {
-    if (L.sp.op == OL_OP_CUMULANT) {
+    if (L.sp.op == OL_OP_CUMULANT && L.sp.omega_3 == 1.0f && L.sp.omega_4 == 1.0f) {
+      if (wale) launch_ws<OL_OP_CUMULANT, true, true>(L, n_sm, s);
+      else launch_ws<OL_OP_CUMULANT, false, true>(L, n_sm, s);
+    } else if (L.sp.op == OL_OP_CUMULANT) {
       if (wale) launch_ws<OL_OP_CUMULANT, true>(L, n_sm, s);
       else launch_ws<OL_OP_CUMULANT, false>(L, n_sm, s);
     } else {

@@ -1296,7 +1296,7 @@ struct GlobalOut {
   }
 };
 
-template <int OP, class ST, bool WALE>
+template <int OP, class ST, bool WALE, bool LOW = false>
 __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbase, float (&A)[27],
                                              int b, int t, bool obs, float spg,
                                              const CellAux *aux = nullptr);
@@ -1317,8 +1317,9 @@ __device__ __forceinline__ void watchdog(int32_t *status, float rho) {
 }
 
 // Everything after the pull: bounce-back, moments, sponge, wall model,
-// WALE, collision, forcing and the stores of cell t of block b.
-template <int OP, class ST, bool WALE>
+// WALE, collision, forcing and the stores of cell t of block b.  LOW: the
+// caller knows that omega_3 = omega_4 = 1.
+template <int OP, class ST, bool WALE, bool LOW>
 __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbase, float (&A)[27],
                                              int b, int t, bool obs, float spg,
                                              const CellAux *aux) {
@@ -1403,8 +1404,10 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
       r.omega4_diag = fminf(fmaxf(Av, 0.01f), 2.0f);
     }
     r.limiter = sp.limiter_type;
-    if (sp.omega_3 == 1.0f && sp.omega_4 == 1.0f) collide_cumulant<true>(A, uxe, uye, uze, r);
-    else collide_cumulant<false>(A, uxe, uye, uze, r);
+    if (LOW || (sp.omega_3 == 1.0f && sp.omega_4 == 1.0f))
+      collide_cumulant<true>(A, uxe, uye, uze, r);
+    else
+      collide_cumulant<false>(A, uxe, uye, uze, r);
     if (sp.limiter_type == OL_LIMITER_POSITIVITY) {
       float fmin = A[0];
 #pragma unroll

@@ -345,7 +345,10 @@ __device__ __forceinline__ float ws_wale(const float *V, int t, float c_wale) {
 // Both operators: the regularized-BGK update needs fewer registers than the
 // cumulant one; its levels took 335 us per coarse step of a 2-level sphere of
 // 32 cells with one CTA per block and 202 us here.
-template <int OP, bool WALE, bool BATCHED>
+// LOW: a level (not a pool, whose items differ) with omega_3 = omega_4 = 1; the
+// general update left out of the kernel's code saves instruction fetches (766 ->
+// 758 us per coarse step of cube_3lvl).
+template <int OP, bool WALE, bool BATCHED, bool LOW = false>
 __global__ void __launch_bounds__(kWsThreads, 1)
     k_sc_ws(const __grid_constant__ LevelDev L0, const LevelDev *__restrict__ descs,
             const WorkItem *__restrict__ items, int n_items, const uint32_t *__restrict__ tab,
@@ -476,7 +479,7 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     if ((t & 31) == 0) mbar_arrive(lfree + bi);
     // item j+1's out-of-block values, in flight while item j collides
     if (j + 1 < cnt) load(j + 1);
-    collide_cell<OP, StoreF32, WALE>(L, nb, A, b, t, obs, spg, &aux);
+    collide_cell<OP, StoreF32, WALE, LOW>(L, nb, A, b, t, obs, spg, &aux);
   }
 }
 
