@@ -130,8 +130,9 @@ __global__ void __launch_bounds__(kWsThreads, 1)
   // per buffer: "landed" (bulk bytes plus the producer's arrival), "free"
   // (one arrival per consumer warp); block j uses buffer j & 1, and its
   // (j >> 1)-th phase of each
-  __shared__ __align__(8) uint64_t bars[4];
+  __shared__ __align__(8) uint64_t bars[5];
   uint64_t *const landed = &bars[0], *const lfree = &bars[2];
+  uint64_t *const ready = &bars[4];  // blocks 0 and 1 are described
   uint2 *const tabs = (uint2 *)(tw_smem + kTwTab);
   const int t = threadIdx.x;
   const int n = D.n_blocks;
@@ -142,10 +143,10 @@ __global__ void __launch_bounds__(kWsThreads, 1)
       mbar_init(landed + i, 1);
       mbar_init(lfree + i, BCELLS / 32);
     }
+    mbar_init(ready, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   const bool wide = ws_wide(D.dstride);
-  ws_load_table(tabs, tab, D.dstride, t);
   __syncthreads();
 
   if (t >= BCELLS) {
@@ -168,6 +169,7 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     };
     fetch(0);
     if (cnt > 1) fetch(1);
+    if (lane == 0) mbar_arrive(ready);
     int j = 0;
     for (; j < cnt; ++j) {
       const int r = j & (kTwRing - 1), bi = j & 1;
@@ -193,17 +195,22 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     ws_halo_load((const float *)D.g_in, D.dstride, wide, ghost_row_of(D, blk[r]), nbb[r], t, tabs,
                  h);
   };
+  // the prologue runs beside the first landing (ws.cuh)
+  ws_load_table(tabs, tab, D.dstride, t);
+  consumer_sync_and(1);
+  const bool described = mbar_wait(ready, 0, fault, kWsFaultConsumerWait);
+  if (described) load(0);
   for (int j = 0; j < cnt; ++j) {
     const int r = j & (kTwRing - 1), bi = j & 1;
     unsigned char *const buf = tw_smem + bi * kTwBuf;
     float *const F = (float *)(buf + kTwS);
-    const bool ok = mbar_wait(landed + bi, (j >> 1) & 1, fault, kWsFaultConsumerWait);
+    const bool ok =
+        described && mbar_wait(landed + bi, (j >> 1) & 1, fault, kWsFaultConsumerWait);
     const int *nbase = nbb[r];
     const int b = blk[r];
     float ux = 0.0f, uy = 0.0f, uz = 0.0f, spg = 0.0f;
     bool obs = false;
     if (ok) {
-      if (j == 0) load(0);
       ws_halo_store(F, nbase, t, tabs, h, absent[r] && !ghost_row_of(D, b),
                     [&](int k, int x, int y, int z) {
                       return pull_boundary_thermal<StoreF32>(D, k, b, x, y, z);

@@ -174,9 +174,13 @@ __device__ __forceinline__ void bulk_copy(void *dst, const void *src, uint32_t b
 
 // Loader table into shared memory with the plane offsets of this launch:
 // tabs[i] = {k * dstride + source cell (mod 2^32), dir | slot << 5 | index << 20}.
+// (by the consumers, while the producer starts the first copies).
 __device__ __forceinline__ void ws_load_table(uint2 *tabs, const uint32_t *__restrict__ tab,
                                               int64_t dstride, int t) {
-  for (int i = t; i < kHaloEntries; i += kWsThreads) {
+#pragma unroll
+  for (int m = 0; m < (kHaloEntries + BCELLS - 1) / BCELLS; ++m) {
+    const int i = t + BCELLS * m;
+    if (i >= kHaloEntries) break;
     const uint2 e = __ldg((const uint2 *)tab + i);
     tabs[i] = make_uint2((e.x >> 9) * (uint32_t)dstride + (e.x & 511), e.y);
   }
@@ -359,8 +363,9 @@ __global__ void __launch_bounds__(kWsThreads, 1)
   __shared__ int blk[kWsRing];
   __shared__ const float *grow[kWsRing];  // the item's ghost row (null: none)
   __shared__ int absent[kWsRing];         // some neighbour of the item is absent
-  __shared__ __align__(8) uint64_t bars[4];
+  __shared__ __align__(8) uint64_t bars[5];
   uint64_t *const landed = &bars[0], *const lfree = &bars[2];
+  uint64_t *const ready = &bars[4];  // items 0 and 1 are described
   uint2 *const tabs = (uint2 *)(ws_smem + kWsTab);
   const int t = threadIdx.x;
   const int n = BATCHED ? n_items : L0.n_blocks;
@@ -374,15 +379,15 @@ __global__ void __launch_bounds__(kWsThreads, 1)
       mbar_init(landed + i, 1);            // the producer's expect_tx arrival + the bulk bytes
       mbar_init(lfree + i, BCELLS / 32);   // one arrival per consumer warp
     }
+    mbar_init(ready, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  ws_load_table(tabs, tab, dstride, t);
   __syncthreads();
-  pdl_wait();  // f_in, vel_in, ghost rows: written by the launches before this one
 
   if (t >= BCELLS) {
     // ------------------------------------------------------------ producer
     const int lane = t - BCELLS;
+    pdl_wait();  // f_in, vel_in: written by the launches before this one
     // descriptor and neighbour offsets of item p into ring slot p & 7
     auto fetch = [&](int p) {
       const int r = p & (kWsRing - 1);
@@ -414,6 +419,7 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     // item j+1's with item j's, so consumers can load ahead
     fetch(0);
     if (cnt > 1) fetch(1);
+    if (lane == 0) mbar_arrive(ready);
     int j = 0;
     for (; j < cnt; ++j) {
       const int r = j & (kWsRing - 1), bi = j & 1;
@@ -442,12 +448,22 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     ws_halo_load((const float *)L.f_in, dstride, wide, grow[r], nbb[r], t, tabs, h);
     if (WALE) ws_vel_load(L, blk[r], nbb[r], t, hv);
   };
+  // The prologue runs beside the first landing: the table, then item 0's
+  // out-of-block loads as soon as it is described.  With both before or after
+  // the landing a launch took 3 us more (8 steps of the 1024-block sphere 413
+  // -> 381 us; per coarse step of cube_3lvl's 7 launches 758 -> 736 us).
+  ws_load_table(tabs, tab, dstride, t);
+  pdl_wait();
+  consumer_sync_and(1);
+  const bool described = mbar_wait(ready, 0, fault, kWsFaultConsumerWait);
+  if (described) load(0);
   for (int j = 0; j < cnt; ++j) {
     const int r = j & (kWsRing - 1), bi = j & 1;
     unsigned char *const buf = ws_smem + bi * kWsBuf;
     float *const S = (float *)(buf + kWsS);
     float *const V = (float *)(buf + kWsV);
-    const bool ok = mbar_wait(landed + bi, (j >> 1) & 1, fault, kWsFaultConsumerWait);
+    const bool ok =
+        described && mbar_wait(landed + bi, (j >> 1) & 1, fault, kWsFaultConsumerWait);
     const LevelDev &L = BATCHED ? Ls[r] : L0;
     const int *const nb = nbb[r];
     const int b = blk[r];
@@ -455,7 +471,6 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     float spg = 0.0f;
     bool obs = false;
     if (ok) {
-      if (j == 0) load(0);
       ws_halo_store(S, nb, t, tabs, h, absent[r] && !grow[r], [&](int k, int x, int y, int z) {
         return pull_boundary<StoreF32>(L, k, b, x, y, z);
       });
