@@ -32,13 +32,18 @@ __host__ __device__ inline float w_of(int k) {
                  : d2 == 1 ? 2.0f / 27.0f : d2 == 2 ? 1.0f / 54.0f : 1.0f / 216.0f;
 }
 
-// Reciprocal, quotient and square root of positive normal floats without a
-// slow path: the hardware approximation (PTX rcp / rsqrt.approx, documented
-// within about one unit in the last place), then one Newton-Raphson step on
-// an FMA residual (Markstein, IBM J. Res. Dev. 34, 1990), which leaves the
-// result within a hair of half a unit.  The operators `/` and sqrtf compile to
-// a range check and a call for the rare operands, and each such call ends a
-// basic block of the cell update; these stay in its straight line.
+// Reciprocal, quotient and square root without a slow path: the hardware
+// approximation (PTX rcp / rsqrt.approx, documented within about one unit in
+// the last place), then a Newton-Raphson step on an FMA residual (Markstein,
+// IBM J. Res. Dev. 34, 1990).  The operators `/` and sqrtf compile to a range
+// check and a call for the rare operands, and each such call ends a basic
+// block of the cell update; these stay in its straight line.  The results are
+// the correctly rounded ones -- the bits of `/` and sqrtf -- in these ranges:
+//   recip_nr(x)        1e-37 <= x <= 2^126 (0 above; the caller clamps infinity);
+//   quotient_nr(a, b)  quotients and operands within 2^+-100; an infinite
+//                      numerator or denominator gives what `/` gives;
+//   sqrt_nr(x)         1e-30 <= x finite (below, the residual is a denormal);
+//   third_of(x)        1e-30 <= |x| finite.
 __device__ __forceinline__ float recip_approx(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -48,10 +53,14 @@ __device__ __forceinline__ float recip_nr(float x) {
   const float r = recip_approx(x);
   return fmaf(r, fmaf(-x, r, 1.0f), r);
 }
+// (the residual step rounds correctly only from a correctly rounded
+// reciprocal: from the approximation, one quotient in 10^9 came out a bit off)
 __device__ __forceinline__ float quotient_nr(float a, float b) {
-  const float r = recip_approx(b);
+  const float d = fminf(b, 3e38f);
+  const float r = recip_nr(d);
   const float q = a * r;
-  return fmaf(fmaf(-b, q, a), r, q);
+  const float e = fmaf(-d, q, a);
+  return fabsf(q) <= 3.4e38f ? fmaf(e, r, q) : q;
 }
 __device__ __forceinline__ float sqrt_nr(float x) {
   float y;
@@ -59,9 +68,8 @@ __device__ __forceinline__ float sqrt_nr(float x) {
   const float s = x * y;
   return fmaf(fmaf(-s, s, x), 0.5f * y, s);
 }
-// x / 3, correctly rounded for normal results: the product with the rounded
-// third, corrected by the exact remainder (Markstein's theorem for constant
-// divisors).
+// x / 3: the product with the rounded third, corrected by the exact remainder
+// (Markstein's theorem for constant divisors).
 __device__ __forceinline__ float third_of(float x) {
   const float c = 0.333333343f;  // the float nearest 1/3
   const float q = x * c;

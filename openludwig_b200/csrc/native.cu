@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(512, OP == OL_OP_CUMULANT ? 2 : 1)
     const bool miss = load_nbbase_sync(L.nbr, L.nbr_stride, L.block_offset, w.block, t, nbbase);
     stage_flow<ST>(L, nbbase, w.block, t, E, miss, r);
     __syncthreads();
-    stream_collide_cell<OP, ST, WALE>(L, nbbase, E, w.block, t, obs, spg);
+    stream_collide_cell<OP, ST, WALE, pool_sums(OP)>(L, nbbase, E, w.block, t, obs, spg);
     if (DDF) {
       __syncthreads();
       stage_thermal<ST>(D, nbbase, w.block, t, E, L.halo_tab, miss);

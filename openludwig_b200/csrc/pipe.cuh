@@ -111,7 +111,8 @@ __global__ void __launch_bounds__(512, OP == OL_OP_CUMULANT ? 2 : 1)
     __syncthreads();  // staging buffer free
     bool fill = false;
     if (nxt < n) fill = issue_stage_f32(BATCHED ? Ls[sn] : L0, nbb[sn], nblk, t, E, nmiss);
-    collide_cell<OP, StoreF32, WALE>(Lc, nbb[cur], A, blk, t, obs, spg);
+    collide_cell<OP, StoreF32, WALE, false, BATCHED ? pool_sums(OP) : kSumsShort>(
+        Lc, nbb[cur], A, blk, t, obs, spg);
     if (nxt >= n) break;
     if (fill) fill_missing_flow<StoreF32>(BATCHED ? Ls[sn] : L0, nbb[sn], nblk, t, E);
     it = nxt;

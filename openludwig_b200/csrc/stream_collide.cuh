@@ -367,11 +367,31 @@ __device__ __forceinline__ void wall_force(float dist, float rho, float ux, floa
 //   * with omega_3 = omega_4 = 1 (the reference's defaults) every third-order
 //     moment and every C_211 kind is relaxed to exactly zero, so its forward
 //     transform, the fifth-order products and the zero terms of the backward
-//     transform are left out (collide_cumulant<true>).
+//     transform are left out (collide_cumulant<true, ...>).
+//
+// SUMS: the order and rounding of the sums.  kSumsShort is the form above.  The
+// block pool takes the order of the written formulas -- rho and the momentum
+// over the 27 populations in turn, a triple's zeroth moment as (a + b) + c, a
+// product that two terms share rounded on its own -- about 80 additions a cell
+// more.  Its force coefficients are read from the first hundred steps on, while
+// the start's pressure wave still swings the drag through zero; there another
+// rounding of any one term shows at up to 1e-3 of the coefficient vector (5e-3
+// with FP16 storage), so a pool's records compare between builds only where the
+// update rounds alike.  kSumsPool and kSumsPoolWs (k_sc_ws) differ in one place:
+// the latter forms u_z^2 rho once, rounded, for both transforms along z.  What
+// is fused is written out (fmaf, __fmul_rn), so that no compiler's choice
+// enters.  8 steps of a pool of 6 cases: 5404 us, 5335 us with kSumsShort
+// (FP16 storage 6523 and 6438 us).
 // ---------------------------------------------------------------------------
+constexpr int kSumsShort = 0, kSumsPool = 1, kSumsPoolWs = 2;
+// The block pool's form (regularized BGK has one form only).
+constexpr int pool_sums(int op, bool ws = false) {
+  return op != OL_OP_CUMULANT ? kSumsShort : ws ? kSumsPoolWs : kSumsPool;
+}
+template <int SUMS>
 __device__ __forceinline__ void raw_moments(float &a, float &b, float &c) {
   const float m2 = a + c, m1 = c - a;
-  a = b + m2;
+  a = SUMS != kSumsShort ? (a + b) + c : b + m2;
   b = m1;
   c = m2;
 }
@@ -381,27 +401,41 @@ __device__ __forceinline__ void centre(float m0, float &b, float &c, float u) {
   b = fmaf(-u, m0, m1);
   c = fmaf(u * u, m0, fmaf(-2.0f * u, m1, c));
 }
+template <int SUMS>
 __device__ __forceinline__ void chim_fwd(float &a, float &b, float &c, float u) {
-  raw_moments(a, b, c);
+  raw_moments<SUMS>(a, b, c);
   centre(a, b, c, u);
 }
 // (m2 +- m1) / 2 as fma(+-1/2, m1, m2 / 2): the same bits (halving is exact
 // at these magnitudes, so both round the same exact value once), one
 // instruction fewer.
-__device__ __forceinline__ void chim_bwd(float &a, float &b, float &c, float u) {
-  const float m0 = a, m1 = fmaf(u, a, b), m2 = fmaf(u * u, a, fmaf(2.0f * u, b, c));
+__device__ __forceinline__ void chim_bwd_from(float &a, float &b, float &c, float m0, float m1,
+                                              float m2) {
   const float h = 0.5f * m2;
   c = fmaf(0.5f, m1, h);
   a = fmaf(-0.5f, m1, h);
-  b = m0 - m2;
+  b = __fsub_rn(m0, m2);
 }
-// The same for a zero first moment ...
+__device__ __forceinline__ void chim_bwd(float &a, float &b, float &c, float u) {
+  chim_bwd_from(a, b, c, a, fmaf(u, a, b), fmaf(u * u, a, fmaf(2.0f * u, b, c)));
+}
+// The same with the second moment given as a factor of r ...
+__device__ __forceinline__ void chim_bwd_r(float &a, float &b, float &c, float u, float r) {
+  const float m2 = fmaf(u * u, a, fmaf(r, c, __fmul_rn(2.0f * u, b)));
+  chim_bwd_from(a, b, c, a, fmaf(u, a, b), m2);
+}
+// ... for a zero first moment ...
 __device__ __forceinline__ void chim_bwd_b0(float &a, float &b, float &c, float u) {
-  const float m0 = a, m1 = u * a, m2 = fmaf(u * u, a, c);
-  const float h = 0.5f * m2;
-  c = fmaf(0.5f, m1, h);
-  a = fmaf(-0.5f, m1, h);
-  b = m0 - m2;
+  chim_bwd_from(a, b, c, a, u * a, fmaf(u * u, a, c));
+}
+// ... for the line of rho with u^2 rho rounded (kSumsPoolWs; forward, its first
+// moment is not used) ...
+__device__ __forceinline__ void chim_fwd_rho(float &a, float &b, float &c, float u) {
+  raw_moments<kSumsPoolWs>(a, b, c);
+  c = __fadd_rn(fmaf(-2.0f * u, b, c), __fmul_rn(u * u, a));
+}
+__device__ __forceinline__ void chim_bwd_rho(float &a, float &b, float &c, float u) {
+  chim_bwd_from(a, b, c, a, u * a, __fadd_rn(c, __fmul_rn(u * u, a)));
 }
 // ... and for a triple that holds a first moment only.
 __device__ __forceinline__ void chim_bwd_b(float &a, float &b, float &c, float u) {
@@ -418,7 +452,7 @@ struct CumulantRates {
 
 // A holds raw x-moments on entry (raw_moments over the consecutive triples)
 // and populations on exit.  LOW: omega3 == omega4 == 1.
-template <bool LOW>
+template <bool LOW, int SUMS>
 __device__ __forceinline__ void collide_cumulant(float (&A)[27], float ux, float uy, float uz,
                                                  const CumulantRates &r) {
   // forward: x (consecutive triples), then y (stride 3), then z (stride 9)
@@ -428,27 +462,32 @@ __device__ __forceinline__ void collide_cumulant(float (&A)[27], float ux, float
   for (int zz = 0; zz < 3; ++zz)
 #pragma unroll
     for (int a = 0; a < 3; ++a)
-      chim_fwd(A[a + 9 * zz], A[a + 3 + 9 * zz], A[a + 6 + 9 * zz], uy);
+      chim_fwd<SUMS>(A[a + 9 * zz], A[a + 3 + 9 * zz], A[a + 6 + 9 * zz], uy);
+  if constexpr (SUMS == kSumsPoolWs) chim_fwd_rho(A[0], A[9], A[18], uz);
+  else chim_fwd<SUMS>(A[0], A[9], A[18], uz);
 #pragma unroll
-  for (int i = 0; i < 9; ++i) chim_fwd(A[i], A[i + 9], A[i + 18], uz);
+  for (int i = 1; i < 9; ++i) chim_fwd<SUMS>(A[i], A[i + 9], A[i + 18], uz);
 
   const float k000 = A[0];
   const float inv_r = recip_nr(fmaxf(k000, 0.01f));
   // index of central moment (a,b,c) = a + 3b + 9c
-  const float c200 = A[2] * inv_r, c020 = A[6] * inv_r, c002 = A[18] * inv_r;
-  const float c110 = A[4] * inv_r, c101 = A[10] * inv_r, c011 = A[12] * inv_r;
-  const float c220n = A[8] * inv_r, c202n = A[20] * inv_r, c022n = A[24] * inv_r;
-
-  const float C220 = c220n - c200 * c020 - 2.0f * c110 * c110;
-  const float C202 = c202n - c200 * c002 - 2.0f * c101 * c101;
-  const float C022 = c022n - c020 * c002 - 2.0f * c011 * c011;
+  auto central = [&](float k) { return __fmul_rn(k, inv_r); };
+  const float c200 = central(A[2]), c020 = central(A[6]), c002 = central(A[18]);
+  const float c110 = central(A[4]), c101 = central(A[10]), c011 = central(A[12]);
+  // cumulant C of a fourth-order moment k: k / r - p q - 2 s t
+  auto cumulant = [&](float k, float p, float q, float s, float t) {
+    return fmaf(-2.0f * s, t, fmaf(k, inv_r, -__fmul_rn(p, q)));
+  };
+  const float C220 = cumulant(A[8], c200, c020, c110, c110);
+  const float C202 = cumulant(A[20], c200, c002, c101, c101);
+  const float C022 = cumulant(A[24], c020, c002, c011, c011);
 
   const float cs2 = 0.333333333f;
   const float om1 = r.omega1, omb = r.omega_bulk;
   const float Dtr = c200 + c020 + c002;
-  const float Dtr_s = (1.0f - omb) * Dtr + omb * (3.0f * cs2);
-  const float D1s = (1.0f - om1) * (c200 - c020);
-  const float D2s = (1.0f - om1) * (c200 - c002);
+  const float Dtr_s = fmaf(1.0f - omb, Dtr, omb * (3.0f * cs2));
+  const float D1s = __fmul_rn(1.0f - om1, c200 - c020);
+  const float D2s = __fmul_rn(1.0f - om1, c200 - c002);
   const float c200s = third_of(Dtr_s + D1s + D2s);
   const float c020s = third_of(Dtr_s - 2.0f * D1s + D2s);
   const float c002s = third_of(Dtr_s + D1s - 2.0f * D2s);
@@ -456,18 +495,19 @@ __device__ __forceinline__ void collide_cumulant(float (&A)[27], float ux, float
   float c101s = (1.0f - om1) * c101;
   float c011s = (1.0f - om1) * c011;
   if (r.limiter == OL_LIMITER_FACTORED) {
-    // (a floor far below any product's rounding keeps the root defined)
-    const float b110 = sqrt_nr(fmaxf(c200s * c020s, 1e-36f));
-    const float b101 = sqrt_nr(fmaxf(c200s * c002s, 1e-36f));
-    const float b011 = sqrt_nr(fmaxf(c020s * c002s, 1e-36f));
+    auto root = [](float v) { return v > 1e-30f ? sqrt_nr(v) : 0.0f; };
+    const float b110 = root(c200s * c020s);
+    const float b101 = root(c200s * c002s);
+    const float b011 = root(c020s * c002s);
     c110s = fminf(fmaxf(c110s, -b110), b110);
     c101s = fminf(fmaxf(c101s, -b101), b101);
     c011s = fminf(fmaxf(c011s, -b011), b011);
   }
   const float o4d = 1.0f - r.omega4_diag;
-  const float C220s = o4d * C220, C202s = o4d * C202, C022s = o4d * C022;
+  const float C220s = __fmul_rn(o4d, C220), C202s = __fmul_rn(o4d, C202),
+              C022s = __fmul_rn(o4d, C022);
   const float rr = k000;
-  if constexpr (LOW) {
+  if constexpr (LOW && SUMS == kSumsShort) {
     // e = C + 2 c^2 of each pair; t = 2 c110 c101 is shared by 211 and 222
     const float e220 = fmaf(2.0f * c110s, c110s, C220s);
     const float e202 = fmaf(2.0f * c101s, c101s, C202s);
@@ -481,14 +521,68 @@ __device__ __forceinline__ void collide_cumulant(float (&A)[27], float ux, float
     const float c112s = fmaf(c002s, c110s, 2.0f * c101s * c011s);
     const float c222s =
         fmaf(c002s, c220s, fmaf(c200s, e022, fmaf(c020s, e202, 4.0f * t * c011s)));
-    A[0] = rr;
-    A[2] = rr * c200s; A[6] = rr * c020s; A[18] = rr * c002s;
-    A[4] = rr * c110s; A[10] = rr * c101s; A[12] = rr * c011s;
     A[8] = rr * c220s; A[20] = rr * c202s; A[24] = rr * c022s;
     A[14] = rr * c211s; A[16] = rr * c121s; A[22] = rr * c112s;
     A[26] = rr * c222s;
-    // backward z: (a, b) lines; odd total order is zero
-    chim_bwd_b0(A[0], A[9], A[18], uz);
+  } else {
+    const float p = __fmul_rn(c200s, c020s), x = __fmul_rn(c200s, c011s),
+                y = __fmul_rn(c020s, c101s), z = __fmul_rn(c002s, c110s);
+    const float c220s = fmaf(2.0f * c110s, c110s, __fadd_rn(C220s, p));
+    const float c202s = fmaf(2.0f * c101s, c101s, fmaf(c200s, c002s, C202s));
+    const float c022s = fmaf(2.0f * c011s, c011s, fmaf(c020s, c002s, C022s));
+    float c211s = x, c121s = y, c112s = z;
+    // 222: the terms in C, those in third-order moments, the rest
+    float c222s = fmaf(c002s, C220s, fmaf(c020s, C202s, __fmul_rn(c200s, C022s)));
+    const float q = fmaf(z, c110s, fmaf(y, c101s, __fmul_rn(x, c011s)));
+    const float rest = fmaf(__fmul_rn(8.0f * c110s, c101s), c011s, fmaf(p, c002s, 2.0f * q));
+    if constexpr (!LOW) {
+      const float o3 = 1.0f - r.omega3, o4 = 1.0f - r.omega4;
+      auto third_order = [&](float k) { return __fmul_rn(o3, central(k)); };
+      const float c210s = third_order(A[5]), c120s = third_order(A[7]);
+      const float c201s = third_order(A[11]), c021s = third_order(A[15]);
+      const float c102s = third_order(A[19]), c012s = third_order(A[21]);
+      const float c111s = third_order(A[13]);
+      const float C211s = __fmul_rn(o4, cumulant(A[14], c200, c011, c110, c101));
+      const float C121s = __fmul_rn(o4, cumulant(A[16], c020, c101, c110, c011));
+      const float C112s = __fmul_rn(o4, cumulant(A[22], c002, c110, c101, c011));
+      c211s = __fadd_rn(C211s, c211s);
+      c121s = __fadd_rn(C121s, c121s);
+      c112s = __fadd_rn(C112s, c112s);
+      const float c221s =
+          fmaf(2.0f * c011s, c210s,
+               fmaf(2.0f * c101s, c120s,
+                    fmaf(4.0f * c110s, c111s, fmaf(c020s, c201s, __fmul_rn(c200s, c021s)))));
+      const float c212s =
+          fmaf(2.0f * c011s, c201s,
+               fmaf(4.0f * c101s, c111s,
+                    fmaf(2.0f * c110s, c102s, fmaf(c002s, c210s, __fmul_rn(c200s, c012s)))));
+      const float c122s =
+          fmaf(2.0f * c101s, c021s,
+               fmaf(4.0f * c011s, c111s,
+                    fmaf(2.0f * c110s, c012s, fmaf(c002s, c120s, __fmul_rn(c020s, c102s)))));
+      c222s = fmaf(4.0f, fmaf(c011s, C211s, fmaf(c110s, C112s, __fmul_rn(c101s, C121s))), c222s);
+      const float t = fmaf(c120s, c102s, fmaf(c201s, c021s, __fmul_rn(c210s, c012s)));
+      c222s = __fadd_rn(c222s, fmaf(4.0f * c111s, c111s, 2.0f * t));
+      A[5] = rr * c210s; A[7] = rr * c120s; A[11] = rr * c201s; A[15] = rr * c021s;
+      A[13] = rr * c111s;
+      A[17] = rr * c221s;
+      A[19] = c102s; A[21] = c012s; A[23] = c212s; A[25] = c122s;  // (chim_bwd_r)
+    }
+    c211s = fmaf(2.0f * c110s, c101s, c211s);
+    c121s = fmaf(2.0f * c110s, c011s, c121s);
+    c112s = fmaf(2.0f * c101s, c011s, c112s);
+    c222s = __fadd_rn(c222s, rest);
+    const float s = LOW ? rr : 1.0f;
+    A[8] = rr * c220s; A[14] = rr * c211s; A[16] = rr * c121s;
+    A[20] = s * c202s; A[22] = s * c112s; A[24] = s * c022s; A[26] = s * c222s;
+  }
+  A[0] = rr;
+  A[2] = rr * c200s; A[6] = rr * c020s; A[18] = rr * c002s;
+  A[4] = rr * c110s; A[10] = rr * c101s; A[12] = rr * c011s;
+  // backward z: (a, b) lines
+  if constexpr (SUMS == kSumsPoolWs) chim_bwd_rho(A[0], A[9], A[18], uz);
+  else chim_bwd_b0(A[0], A[9], A[18], uz);
+  if constexpr (LOW) {  // odd total order is zero
     chim_bwd_b0(A[2], A[11], A[20], uz);
     chim_bwd_b0(A[4], A[13], A[22], uz);
     chim_bwd_b0(A[6], A[15], A[24], uz);
@@ -498,53 +592,9 @@ __device__ __forceinline__ void collide_cumulant(float (&A)[27], float ux, float
     chim_bwd_b(A[5], A[14], A[23], uz);
     chim_bwd_b(A[7], A[16], A[25], uz);
   } else {
-    const float c210 = A[5] * inv_r, c120 = A[7] * inv_r, c201 = A[11] * inv_r;
-    const float c021 = A[15] * inv_r, c102 = A[19] * inv_r, c012 = A[21] * inv_r;
-    const float c111 = A[13] * inv_r;
-    const float c211n = A[14] * inv_r, c121n = A[16] * inv_r, c112n = A[22] * inv_r;
-    const float C211 = c211n - c200 * c011 - 2.0f * c110 * c101;
-    const float C121 = c121n - c020 * c101 - 2.0f * c110 * c011;
-    const float C112 = c112n - c002 * c110 - 2.0f * c101 * c011;
-    const float o3 = 1.0f - r.omega3;
-    const float c210s = o3 * c210, c120s = o3 * c120, c201s = o3 * c201;
-    const float c021s = o3 * c021, c102s = o3 * c102, c012s = o3 * c012;
-    const float c111s = o3 * c111;
-    const float o4 = 1.0f - r.omega4;
-    const float C211s = o4 * C211, C121s = o4 * C121, C112s = o4 * C112;
-
-    const float c220s = C220s + c200s * c020s + 2.0f * c110s * c110s;
-    const float c202s = C202s + c200s * c002s + 2.0f * c101s * c101s;
-    const float c022s = C022s + c020s * c002s + 2.0f * c011s * c011s;
-    const float c211s = C211s + c200s * c011s + 2.0f * c110s * c101s;
-    const float c121s = C121s + c020s * c101s + 2.0f * c110s * c011s;
-    const float c112s = C112s + c002s * c110s + 2.0f * c101s * c011s;
-    const float c221s = c200s * c021s + c020s * c201s + 4.0f * c110s * c111s +
-                        2.0f * c101s * c120s + 2.0f * c011s * c210s;
-    const float c212s = c200s * c012s + c002s * c210s + 2.0f * c110s * c102s +
-                        4.0f * c101s * c111s + 2.0f * c011s * c201s;
-    const float c122s = c020s * c102s + c002s * c120s + 2.0f * c110s * c012s +
-                        4.0f * c011s * c111s + 2.0f * c101s * c021s;
-    float c222s = c200s * C022s + c020s * C202s + c002s * C220s +
-                  4.0f * (c110s * C112s + c101s * C121s + c011s * C211s);
-    c222s += 2.0f * (c210s * c012s + c201s * c021s + c120s * c102s) + 4.0f * c111s * c111s;
-    c222s += c200s * c020s * c002s +
-             2.0f * (c200s * c011s * c011s + c020s * c101s * c101s + c002s * c110s * c110s) +
-             8.0f * c110s * c101s * c011s;
-
-    A[0] = rr;
-    A[1] = 0.0f; A[3] = 0.0f; A[9] = 0.0f;
-    A[2] = rr * c200s; A[6] = rr * c020s; A[18] = rr * c002s;
-    A[4] = rr * c110s; A[10] = rr * c101s; A[12] = rr * c011s;
-    A[5] = rr * c210s; A[7] = rr * c120s; A[11] = rr * c201s;
-    A[15] = rr * c021s; A[19] = rr * c102s; A[21] = rr * c012s;
-    A[13] = rr * c111s;
-    A[8] = rr * c220s; A[20] = rr * c202s; A[24] = rr * c022s;
-    A[14] = rr * c211s; A[16] = rr * c121s; A[22] = rr * c112s;
-    A[17] = rr * c221s; A[23] = rr * c212s; A[25] = rr * c122s;
-    A[26] = rr * c222s;
-    // backward z
+    A[1] = 0.0f; A[3] = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 9; ++i) chim_bwd(A[i], A[i + 9], A[i + 18], uz);
+    for (int i = 1; i < 9; ++i) chim_bwd_r(A[i], A[i + 9], A[i + 18], uz, rr);
   }
   // backward y, then x
 #pragma unroll
@@ -1296,18 +1346,18 @@ struct GlobalOut {
   }
 };
 
-template <int OP, class ST, bool WALE, bool LOW = false>
+template <int OP, class ST, bool WALE, bool LOW = false, int SUMS = kSumsShort>
 __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbase, float (&A)[27],
                                              int b, int t, bool obs, float spg,
                                              const CellAux *aux = nullptr);
 
-template <int OP, class ST, bool WALE>
+template <int OP, class ST, bool WALE, int SUMS = kSumsShort>
 __device__ __forceinline__ void stream_collide_cell(const LevelDev &L, const int *nbbase,
                                                     const float *E, int b, int t, bool obs,
                                                     float spg) {
   float A[27];
   load_pulls(E, t, A);
-  collide_cell<OP, ST, WALE>(L, nbbase, A, b, t, obs, spg);
+  collide_cell<OP, ST, WALE, false, SUMS>(L, nbbase, A, b, t, obs, spg);
 }
 
 // Device watchdog of the native path: non-finite or vanishing density.
@@ -1319,7 +1369,7 @@ __device__ __forceinline__ void watchdog(int32_t *status, float rho) {
 // Everything after the pull: bounce-back, moments, sponge, wall model,
 // WALE, collision, forcing and the stores of cell t of block b.  LOW: the
 // caller knows that omega_3 = omega_4 = 1.
-template <int OP, class ST, bool WALE, bool LOW>
+template <int OP, class ST, bool WALE, bool LOW, int SUMS>
 __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbase, float (&A)[27],
                                              int b, int t, bool obs, float spg,
                                              const CellAux *aux) {
@@ -1340,14 +1390,25 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
     out.template f_all<true>(A);
     return;
   }
-  // A becomes the raw x-moments (m0, m1, m2) of each (y, z) triple
+  if constexpr (SUMS != kSumsShort) {
+    rho = jx = jy = jz = 0.0f;
 #pragma unroll
-  for (int i = 0; i < 9; ++i) raw_moments(A[3 * i], A[3 * i + 1], A[3 * i + 2]);
-  const float s0 = A[0] + A[3] + A[6], s1 = A[9] + A[12] + A[15], s2 = A[18] + A[21] + A[24];
-  rho = s0 + s1 + s2;
-  jx = (A[1] + A[4] + A[7]) + (A[10] + A[13] + A[16]) + (A[19] + A[22] + A[25]);
-  jy = (A[6] - A[0]) + (A[15] - A[9]) + (A[24] - A[18]);
-  jz = s2 - s0;
+    for (int k = 0; k < 27; ++k) {
+      rho += A[k];
+      if (cx_of(k) == 1) jx += A[k]; else if (cx_of(k) == -1) jx -= A[k];
+      if (cy_of(k) == 1) jy += A[k]; else if (cy_of(k) == -1) jy -= A[k];
+      if (cz_of(k) == 1) jz += A[k]; else if (cz_of(k) == -1) jz -= A[k];
+    }
+  } else {
+    // A becomes the raw x-moments (m0, m1, m2) of each (y, z) triple
+#pragma unroll
+    for (int i = 0; i < 9; ++i) raw_moments<kSumsShort>(A[3 * i], A[3 * i + 1], A[3 * i + 2]);
+    const float s0 = A[0] + A[3] + A[6], s1 = A[9] + A[12] + A[15], s2 = A[18] + A[21] + A[24];
+    rho = s0 + s1 + s2;
+    jx = (A[1] + A[4] + A[7]) + (A[10] + A[13] + A[16]) + (A[19] + A[22] + A[25]);
+    jy = (A[6] - A[0]) + (A[15] - A[9]) + (A[24] - A[18]);
+    jz = s2 - s0;
+  }
   // device watchdog (native path): report, never trap
   if (L.status) watchdog(L.status, rho);
   rho = fminf(fmaxf(rho, 0.01f), 3e38f);
@@ -1366,11 +1427,15 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
         for (int j = 0; j < 3; ++j)
           ft[j] = feq_auto(1.0f, sp.u_inlet, 0.0f, 0.0f, w_of(3 * i + j), (float)cx_of(3 * i + j),
                            (float)cy_of(3 * i + j), (float)cz_of(3 * i + j), sp.compressible_corr);
-        raw_moments(ft[0], ft[1], ft[2]);
+        if constexpr (SUMS == kSumsShort) raw_moments<kSumsShort>(ft[0], ft[1], ft[2]);
 #pragma unroll
         for (int j = 0; j < 3; ++j) A[3 * i + j] = A[3 * i + j] * (1.0f - spg) + ft[j] * spg;
       }
     }
+  }
+  if constexpr (SUMS != kSumsShort) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) raw_moments<SUMS>(A[3 * i], A[3 * i + 1], A[3 * i + 2]);
   }
   float Fx = 0.0f, Fy = 0.0f, Fz = 0.0f;
   if (sp.wall_model_active == 1 && L.wall_dist)
@@ -1405,9 +1470,9 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
     }
     r.limiter = sp.limiter_type;
     if (LOW || (sp.omega_3 == 1.0f && sp.omega_4 == 1.0f))
-      collide_cumulant<true>(A, uxe, uye, uze, r);
+      collide_cumulant<true, SUMS>(A, uxe, uye, uze, r);
     else
-      collide_cumulant<false>(A, uxe, uye, uze, r);
+      collide_cumulant<false, SUMS>(A, uxe, uye, uze, r);
     if (sp.limiter_type == OL_LIMITER_POSITIVITY) {
       float fmin = A[0];
 #pragma unroll

@@ -494,7 +494,8 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     if ((t & 31) == 0) mbar_arrive(lfree + bi);
     // item j+1's out-of-block values, in flight while item j collides
     if (j + 1 < cnt) load(j + 1);
-    collide_cell<OP, StoreF32, WALE, LOW>(L, nb, A, b, t, obs, spg, &aux);
+    collide_cell<OP, StoreF32, WALE, LOW, BATCHED ? pool_sums(OP, true) : kSumsShort>(
+        L, nb, A, b, t, obs, spg, &aux);
   }
 }
 
