@@ -1411,8 +1411,8 @@ __device__ __forceinline__ void collide_cell(const LevelDev &L, const int *nbbas
   }
   // device watchdog (native path): report, never trap
   if (L.status) watchdog(L.status, rho);
-  rho = fminf(fmaxf(rho, 0.01f), 3e38f);
-  const float inv_rho = recip_nr(rho);
+  rho = fmaxf(rho, 0.01f);  // (an infinite density is stored as such)
+  const float inv_rho = recip_nr(fminf(rho, 3e38f));
   float ux = jx * inv_rho, uy = jy * inv_rho, uz = jz * inv_rho;
   if (spg > 0.0f) {
     rho = rho * (1.0f - spg) + 1.0f * spg;

@@ -5,6 +5,7 @@
   one-CTA-per-block and the warp-specialised kernel, against the oracle: the
   single-step bar of test_gpu_stream_collide (2e-6 absolute, 1e-5 relative L2:
   a few rounding errors of the largest population);
+* a density beyond the float range is stored as infinity, not as a large number;
 * the ghost pass on a domain whose size is no multiple of a block, where a
   group of ring positions lies partly outside it: bitwise the in-staging fill."""
 import numpy as np
@@ -64,6 +65,25 @@ def test_single_step_matches_oracle(sphere, var, choice, ctas):
                        {name: getattr(inp["sp"], name) for name, _ in N.STEP_FIELDS})
     assert max_abs(f, o_f) < 2e-6 and rel_err(f, o_f) < 1e-5
     assert max_abs(r, o_rho) < 2e-6 and max_abs(v, o_vel) < 2e-6
+
+
+@pytest.mark.parametrize("choice", [BLOCK, WS], ids=["block", "ws"])
+@pytest.mark.parametrize("value", [float("inf"), 3.2e38, float("-inf")])
+@pytest.mark.parametrize("op", [0, 1], ids=["cumulant", "bgk"])
+def test_density_out_of_range_is_stored(sphere, op, value, choice):
+    c, mesh, p, hosts = sphere
+    h = hosts[0]
+    st = S.StepSettings(op=op, limiter=1, c_wale=0.5)
+    cells = np.flatnonzero((np.asarray(h.obstacle).reshape(-1) == 0) &
+                           (np.asarray(h.sponge).reshape(-1) == 0))[::97]
+    _kernel(choice)
+    lv = S.upload_level(h, DEV)
+    src = lv.f_temp  # step 1 reads the second buffer
+    src.view(27, -1)[13, torch.from_numpy(cells).to(DEV)] = value  # the rest population
+    S.recursive_step([lv], st, 0, 1, None, 0.0, 0.05, (p.nx_coarse, p.ny_coarse, p.nz_coarse))
+    got = lv.rho.cpu().numpy()[cells]
+    # (the other 26 populations add 0.7, far below the last bit of 3.2e38)
+    assert np.array_equal(got, np.full(len(cells), np.float32(max(value, 0.01))))
 
 
 @pytest.mark.parametrize("cut", [(0, 0, 0), (3, 0, 0), (1, 2, 5)])
