@@ -42,6 +42,15 @@ def build(force: bool = False) -> Path:
     return LIB_PATH
 
 
+def build_probe() -> Path:
+    """The comparison of the library's device helpers with CUDA's rounded
+    operations (ol_probe_gpu.cu); make decides whether it is up to date."""
+    r = subprocess.run(["make", "-C", str(HERE), "probe"], capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"helper probe build failed:\n{r.stdout}\n{r.stderr}")
+    return HERE / "_build" / "libolprobe_gpu.so"
+
+
 def lib() -> C.CDLL:
     global _lib
     if _lib is None:
