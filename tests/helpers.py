@@ -28,16 +28,47 @@ def small_sphere_case(resolution: int = 8, levels: int = 1, bouzidi: bool = True
     return c, mesh, p, hosts
 
 
-def interior_refined_case():
+def interior_refined_case(**kw):
     """Two-level cube (48 finest cells, Re 1.6e5, alpha 3.2, beta -1.9) whose
     refined level lies inside the domain: all its absent-neighbour values
     are coarse-to-fine (4096 fine blocks, 1352 at the interface)."""
     m = workloads.MixCase("cube", 48, 2, 158378.0, 3.18, -1.94)
     c, mesh = workloads.mix_case_config(m)
+    return _built(c, mesh, kw)
+
+
+def interior_three_level_case(**kw):
+    """The three-level cube at 48 finest cells: levels 2 and 3 (1728 and 3584
+    blocks) both lie inside the domain, so each child reads its parent."""
+    c, mesh = workloads.cube_3lvl()
+    c.surface_resolution = 48
+    return _built(c, mesh, kw)
+
+
+def _built(c, mesh, kw):
     c.ramp_steps = 0
+    for k, v in kw.items():
+        setattr(c, k, v)
     p = scaling.compute_domain_from_mesh(c, mesh.min_bounds, mesh.max_bounds)
     hosts = domain.setup_multilevel_domain(c, mesh, p)
     return c, mesh, p, hosts
+
+
+def absent_neighbours(h, dims):
+    """How many absent neighbours of a level's blocks lie wholly inside the
+    domain (dims: the level's size in cells), partly, and wholly outside."""
+    nb = np.asarray(h.neighbor_table).reshape(27, h.n_blocks)
+    n = np.zeros(3, int)
+    for d in range(27):
+        inside = touching = np.ones(h.n_blocks, bool)
+        for a, m in enumerate((h.map_x, h.map_y, h.map_z)):
+            c = np.asarray(m).astype(int) + d // 3 ** a % 3 - 1
+            inside = inside & (c >= 1) & (c * 8 <= dims[a])
+            touching = touching & (c >= 1) & ((c - 1) * 8 < dims[a])
+        absent = nb[d] <= 0
+        n += [(absent & inside).sum(), (absent & touching & ~inside).sum(),
+              (absent & ~touching).sum()]
+    return tuple(int(x) for x in n)
 
 
 def lattice():

@@ -6,12 +6,13 @@
   single-step bar of test_gpu_stream_collide (2e-6 absolute, 1e-5 relative L2:
   a few rounding errors of the largest population);
 * a density beyond the float range is stored as infinity, not as a large number;
-* the ghost pass on a domain whose size is no multiple of a block, where a
-  group of ring positions lies partly outside it: bitwise the in-staging fill."""
+* the ghost pass, paired and unpaired, on a refined region inside the domain and
+  on domains whose edge cuts the blocks beyond that region, where a group of
+  ring positions lies partly outside: bitwise the in-staging fill."""
 import numpy as np
 import pytest
 
-from helpers import max_abs, rel_err, small_sphere_case
+from helpers import absent_neighbours, interior_refined_case, max_abs, rel_err, small_sphere_case
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -86,23 +87,43 @@ def test_density_out_of_range_is_stored(sphere, op, value, choice):
     assert np.array_equal(got, np.full(len(cells), np.float32(max(value, 0.01))))
 
 
-@pytest.mark.parametrize("cut", [(0, 0, 0), (3, 0, 0), (1, 2, 5)])
+# Level-1 sizes: the refined region of the interior case ends at fine block
+# (20, 18, 18), so fine blocks 21, 19 and 19 beyond it are cut by an edge at 2, 4
+# and 6 of their 8 cells.
+DOMAINS = {"edge": None, "inside": (0, 0, 0), "cut_x": (81, 0, 0), "cut_xyz": (81, 74, 75),
+           "cut_yz": (0, 73, 73)}
+
+
+@pytest.mark.parametrize("where", DOMAINS)
 @pytest.mark.parametrize("ddf", [False, True], ids=["flow", "thermal"])
-def test_ghost_pass_on_a_ragged_domain(ddf, cut):
+def test_ghost_pass_on_a_ragged_domain(ddf, where):
     kw = dict(compressibility_correction=True, ddf_enabled=True,
               u_target=np.float32(0.1)) if ddf else {}
-    c, mesh, p, hosts = small_sphere_case(resolution=16, levels=2, c_wale=np.float32(0.5), **kw)
+    if where == "edge":  # the refined region reaches the domain's edge on all sides
+        c, mesh, p, hosts = small_sphere_case(resolution=16, levels=2, c_wale=np.float32(0.5), **kw)
+        dims = (p.nx_coarse - 1, p.ny_coarse - 2, p.nz_coarse - 5)
+    else:
+        c, mesh, p, hosts = interior_refined_case(**kw)
+        dims = tuple(d or n for d, n in zip(DOMAINS[where],
+                                            (p.nx_coarse, p.ny_coarse, p.nz_coarse)))
+        inside, partly, outside = absent_neighbours(hosts[1], [2 * d for d in dims])
+        assert inside > 5000 and (partly > 1000) == where.startswith("cut"), (inside, partly)
     st = S.StepSettings.from_config(c, False)
-    dims = tuple(d - x for d, x in zip((p.nx_coarse, p.ny_coarse, p.nz_coarse), cut))
     runs = []
-    for ghost in (True, False):
-        levels = [S.upload_level(h, DEV, ddf=ddf, ghost=ghost) for h in hosts]
+    for kind in ("paired", "unpaired", "none"):
+        levels = [S.upload_level(h, DEV, ddf=ddf, ghost=kind != "none") for h in hosts]
+        if kind == "unpaired":
+            for lv in levels:
+                lv.ghost2 = lv.ghost_g2 = None
         for t in range(1, 5):
             S.recursive_step(levels, st, 0, t, None, 0.0, 0.1 if ddf else 0.05, dims)
         torch.cuda.synchronize()
         runs.append(levels)
-    for a, b in zip(*runs):
-        assert torch.equal(a.f, b.f) and torch.equal(a.f_temp, b.f_temp)
-        assert torch.equal(a.rho, b.rho) and torch.equal(a.vel, b.vel)
-        if ddf:
-            assert torch.equal(a.g, b.g) and torch.equal(a.g_temp, b.g_temp)
+    assert runs[0][1].ghost2 is not None and runs[2][1].ghost is None
+    for other in runs[:2]:
+        for a, b in zip(other, runs[2]):
+            assert torch.equal(a.f, b.f) and torch.equal(a.f_temp, b.f_temp)
+            assert torch.equal(a.rho, b.rho) and torch.equal(a.vel, b.vel)
+            if ddf:
+                assert torch.equal(a.g, b.g) and torch.equal(a.g_temp, b.g_temp)
+                assert torch.equal(a.temperature, b.temperature)
