@@ -6,7 +6,8 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from helpers import small_sphere_case
+from helpers import (absent_neighbours, interior_refined_case, interior_three_level_case,
+                     small_sphere_case)
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -17,27 +18,60 @@ from openludwig_b200 import _native as N  # noqa: E402
 from openludwig_b200 import solver as S  # noqa: E402
 
 DEV = torch.device("cuda:0")
+DDF = dict(compressibility_correction=True, ddf_enabled=True, u_target=np.float32(0.1))
+# "edge": the refined level fills the domain; "interior" (2 levels) and "three":
+# refined levels inside it, whose values come from the parent's state
 CASES = [
-    dict(name="one_level", levels=1),
-    dict(name="refined", levels=2, c_wale=np.float32(0.5), inlet_turbulence_intensity=0.02),
-    dict(name="no_temporal", levels=2, temporal_interpolation=False),
-    dict(name="restriction", levels=2, fine_to_coarse_restriction=True),
-    dict(name="thermal", levels=2, compressibility_correction=True, ddf_enabled=True,
-         u_target=np.float32(0.1), sponge_blend_distributions=True),
+    dict(name="one_level", domain="one"),
+    dict(name="refined", domain="edge", c_wale=np.float32(0.5), inlet_turbulence_intensity=0.02),
+    dict(name="no_temporal", domain="edge", temporal_interpolation=False),
+    dict(name="restriction", domain="edge", fine_to_coarse_restriction=True),
+    dict(name="thermal", domain="edge", sponge_blend_distributions=True, **DDF),
+    dict(name="interior", domain="interior"),
+    dict(name="interior_no_temporal", domain="interior", temporal_interpolation=False),
+    dict(name="interior_no_ghost", domain="interior", ghost=False),
+    dict(name="interior_thermal", domain="interior", **DDF),
+    dict(name="interior_thermal_restriction", domain="interior", fine_to_coarse_restriction=True,
+         **DDF),
+    dict(name="three", domain="three"),
+    dict(name="three_no_temporal_restriction", domain="three", temporal_interpolation=False,
+         fine_to_coarse_restriction=True),
+    dict(name="three_thermal", domain="three", **DDF),
 ]
+
+
+@pytest.fixture(scope="module")
+def built():
+    """A case's domain, built once for all its step counts."""
+    made = {}
+
+    def get(case):
+        if case["name"] not in made:
+            kw = {k: v for k, v in case.items() if k not in ("name", "domain", "ghost")}
+            d = case["domain"]
+            made.clear()  # (one case's domain at a time)
+            made[case["name"]] = (interior_refined_case(**kw) if d == "interior" else
+                                  interior_three_level_case(**kw) if d == "three" else
+                                  small_sphere_case(resolution=8 if d == "one" else 16,
+                                                    levels=1 if d == "one" else 2, **kw))
+        return made[case["name"]]
+    return get
 
 
 @pytest.mark.parametrize("first,steps", [(1, 1), (1, 3), (4, 2)])
 @pytest.mark.parametrize("case", CASES, ids=[c["name"] for c in CASES])
-def test_batch_equals_single_sub_steps(case, first, steps):
-    kw = {k: v for k, v in case.items() if k not in ("name", "levels")}
-    c, mesh, p, hosts = small_sphere_case(resolution=16 if case["levels"] > 1 else 8,
-                                          levels=case["levels"], **kw)
+def test_batch_equals_single_sub_steps(built, case, first, steps):
+    c, mesh, p, hosts = built(case)
     st = S.StepSettings.from_config(c, False)
     dims, u = (p.nx_coarse, p.ny_coarse, p.nz_coarse), float(c.u_target)
+    if case["domain"] in ("interior", "three"):
+        assert len(hosts) == (3 if case["domain"] == "three" else 2)
+        for i, h in enumerate(hosts[1:], 1):
+            assert absent_neighbours(h, [d << i for d in dims])[0] > 5000
     runs = []
     for batch in (False, True):
-        levels = [S.upload_level(h, DEV, ddf=c.ddf_enabled) for h in hosts]
+        levels = [S.upload_level(h, DEV, ddf=c.ddf_enabled, ghost=case.get("ghost"))
+                  for h in hosts]
         if batch:
             S.execute_timestep_batch(levels, st, first, steps, u, dims)
         else:
@@ -45,13 +79,12 @@ def test_batch_equals_single_sub_steps(case, first, steps):
                 S.recursive_step(levels, st, 0, first + k, None, 0.0, u, dims)
         torch.cuda.synchronize()
         runs.append(levels)
-    names = ["f", "f_temp", "rho", "vel", "vel_temp"] + (["g", "g_temp", "temperature"]
-                                                          if c.ddf_enabled else [])
+    names = ["f", "f_temp", "rho", "vel", "vel_temp"]
+    names += ["g", "g_temp", "temperature"] if c.ddf_enabled else []
+    old = ["f_old", "rho_old", "vel_old"] + (["g_old", "temperature_old"] if c.ddf_enabled else [])
     for i, (a, b) in enumerate(zip(*runs)):
-        for n in names:
+        for n in names + (old if i + 1 < len(hosts) and st.use_temporal_interp else []):
             assert torch.equal(getattr(a, n), getattr(b, n)), (i, n)
-        if i + 1 < len(hosts) and st.use_temporal_interp:
-            assert torch.equal(a.f_old, b.f_old) and torch.equal(a.rho_old, b.rho_old)
 
 
 def test_march_reports_bad_arguments():
