@@ -482,12 +482,13 @@ def execute_timestep_batch(levels, s: StepSettings, t_start: int, batch: int, u:
                            domain_dims) -> None:
     """solver_control.jl:199-218, as one library call (ol_march).  Levels that
     keep the reference's post-collision copy, or whose scale is not their
-    place in the list, step through recursive_step."""
+    place in the list, and steps before 0 go through recursive_step."""
     if batch <= 0 or not levels:
         return
-    if any(lv.f_post is not None or lv.host.level_id != i + 1
-           or (s.ddf and (lv.g is None or lv.temperature is None))
-           for i, lv in enumerate(levels)):
+    if t_start < 0 or len(levels) > 16 or any(
+            lv.f_post is not None or lv.host.level_id != i + 1
+            or (s.ddf and (lv.g is None or lv.temperature is None))
+            for i, lv in enumerate(levels)):
         for off in range(batch):
             recursive_step(levels, s, 0, t_start + off, None, 0.0, u, domain_dims)
         return

@@ -58,7 +58,7 @@ def built():
     return get
 
 
-@pytest.mark.parametrize("first,steps", [(1, 1), (1, 3), (4, 2)])
+@pytest.mark.parametrize("first,steps", [(1, 1), (1, 3), (4, 2), (-3, 4)])
 @pytest.mark.parametrize("case", CASES, ids=[c["name"] for c in CASES])
 def test_batch_equals_single_sub_steps(built, case, first, steps):
     c, mesh, p, hosts = built(case)
