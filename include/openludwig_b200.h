@@ -175,13 +175,23 @@ OL_API int ol_pipeline_fault(int32_t *flags);
 
 /* Host copies of the static staging tables (no GPU needed; for checking the
  * kernels' index arithmetic): the staging table of the one-CTA-per-block
- * kernel and the ghost pass, and the loader table of the warp-specialised
- * kernel (out-of-block pulls k | dir << 5 | source cell << 10 | pulling cell
- * << 19, face-halo velocity slots, then the FP32 stage slot of each pull).
+ * kernel and the ghost pass, and the table that the warp-specialised kernels'
+ * loader table is made from (out-of-block pulls k | dir << 5 | source cell << 10
+ * | pulling cell << 19, face-halo velocity slots, then the FP32 stage slot of
+ * each pull).
  * sizes[4] = {halo entries, loader entries, stage plane slots, stage pad}; a
  * table is copied when its buffer is non-NULL and large enough. */
 OL_API int ol_staging_tables(uint32_t *halo, int32_t halo_cap, uint32_t *ws, int32_t ws_cap,
                              int32_t *sizes);
+
+/* The warp-specialised kernels' loader table as they read it, evaluated on the
+ * host by their own index functions (no GPU needed; for checking them): of the
+ * *n entries, rows[4 i ..] = {element offset of the source in 27 planes of
+ * dstride elements (-1: the neighbour is absent), stage slot, neighbour
+ * direction, staging-table index}.  neighbours[27]: first cell of the block in
+ * each direction, < 0: absent.  Copied when rows is non-NULL and cap >= *n. */
+OL_API int ol_ws_loader_sources(int64_t dstride, const int32_t *neighbours, int64_t *rows,
+                                int32_t cap, int32_t *n);
 
 /* Bouzidi interpolated bounce-back (bouzidi_kernel.jl:13-122).  q_map holds
  * IEEE binary16 bit patterns [512*nB*27]; cell_* are the sparse boundary-cell

@@ -514,6 +514,25 @@ extern "C" int ol_staging_tables(uint32_t *halo, int32_t halo_cap, uint32_t *ws,
   return OL_OK;
 }
 
+extern "C" int ol_ws_loader_sources(int64_t dstride, const int32_t *neighbours, int64_t *rows,
+                                    int32_t cap, int32_t *n) {
+  OL_CHECK_ARG(neighbours && n && dstride > 0, "ol_ws_loader_sources: bad arguments");
+  *n = kHaloEntries;
+  if (!rows || cap < kHaloEntries) return OL_OK;
+  const std::vector<uint32_t> tab = build_ws_loader();
+  const bool wide = ws_wide(dstride);
+  for (int i = 0; i < kHaloEntries; ++i) {
+    const uint2 e = ws_entry(make_uint2(tab[2 * i], tab[2 * i + 1]), dstride);
+    const int nb = neighbours[e.y & 31];
+    int64_t *const r = rows + 4 * i;
+    r[0] = nb >= 0 ? ws_source(e, nb, dstride, wide) : -1;
+    r[1] = ws_slot(e);
+    r[2] = e.y & 31;
+    r[3] = e.y >> 20;
+  }
+  return OL_OK;
+}
+
 extern "C" int64_t ol_ghost_floats(int32_t n_blocks) {
   return n_blocks > 0 ? (int64_t)n_blocks * kHaloEntries : 0;
 }

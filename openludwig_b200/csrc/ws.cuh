@@ -62,7 +62,8 @@ constexpr int kWsRing = 8;
 constexpr int kSPad = 72;                         // stage slots before cell 0 (and after 511)
 constexpr int kSPlane = kSPad + BCELLS + kSPad;   // 656 floats = 2624 bytes
 
-// The table ol_staging_tables exports (kWsTableTotal words): the kHaloEntries
+// The table that ol_staging_tables exports (kWsTableTotal words; the loader table
+// below is made from it): the kHaloEntries
 // out-of-block pulls in the order of the staging table (k | dir << 5 | source
 // cell << 10 | destination cell << 19), the kWsVelEntries face-halo velocity
 // entries (face dir | own cell beside the slot << 5), then per pull its stage
@@ -172,24 +173,26 @@ __device__ __forceinline__ void bulk_copy(void *dst, const void *src, uint32_t b
       : "memory");
 }
 
-// Loader table into shared memory with the plane offsets of this launch:
-// tabs[i] = {k * dstride + source cell (mod 2^32), dir | slot << 5 | index << 20}.
-// (by the consumers, while the producer starts the first copies).
+// A loader table entry with the plane offset of this launch:
+// {k * dstride + source cell (mod 2^32), dir | slot << 5 | index << 20}.
+__host__ __device__ __forceinline__ uint2 ws_entry(uint2 e, int64_t dstride) {
+  return make_uint2((e.x >> 9) * (uint32_t)dstride + (e.x & 511), e.y);
+}
+// The table into shared memory (by the consumers, while the producer starts the first copies).
 __device__ __forceinline__ void ws_load_table(uint2 *tabs, const uint32_t *__restrict__ tab,
                                               int64_t dstride, int t) {
 #pragma unroll
   for (int m = 0; m < (kHaloEntries + BCELLS - 1) / BCELLS; ++m) {
     const int i = t + BCELLS * m;
     if (i >= kHaloEntries) break;
-    const uint2 e = __ldg((const uint2 *)tab + i);
-    tabs[i] = make_uint2((e.x >> 9) * (uint32_t)dstride + (e.x & 511), e.y);
+    tabs[i] = ws_entry(__ldg((const uint2 *)tab + i), dstride);
   }
 }
 // Whether the 27 planes reach beyond 32-bit element offsets (over 159 M cells).
-__device__ __forceinline__ bool ws_wide(int64_t dstride) { return 27 * dstride > 0xFFFFFFFFll; }
-__device__ __forceinline__ int ws_slot(uint2 e) { return (e.y >> 5) & 0x7FFF; }
+__host__ __device__ __forceinline__ bool ws_wide(int64_t dstride) { return 27 * dstride > 0xFFFFFFFFll; }
+__host__ __device__ __forceinline__ int ws_slot(uint2 e) { return (e.y >> 5) & 0x7FFF; }
 // Element offset of entry e's source in the neighbour block whose first cell is nb.
-__device__ __forceinline__ int64_t ws_source(uint2 e, int nb, int64_t dstride, bool wide) {
+__host__ __device__ __forceinline__ int64_t ws_source(uint2 e, int nb, int64_t dstride, bool wide) {
   if (!wide) return (int64_t)(e.x + (uint32_t)nb);
   const int k = ws_slot(e) / kSPlane;
   return k * dstride + (uint32_t)(e.x - (uint32_t)k * (uint32_t)dstride) + nb;

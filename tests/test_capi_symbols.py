@@ -88,7 +88,8 @@ def test_ctypes_struct_layouts_match_header(tmp_path):
              "ol_net_force_maps": N.NetForceMaps, "ol_output_level": N.OutputLevel,
              "ol_output_fields": N.OutputFields, "ol_bouzidi_link": N.BouzidiLink,
              "ol_coeff_ref": N.CoeffRef, "ol_serve_rule": N.ServeRule,
-             "ol_serve_result": N.ServeResult, "ol_fe_map_view": N.FeMapView}
+             "ol_serve_result": N.ServeResult, "ol_fe_map_view": N.FeMapView,
+             "ol_march_level": N.MarchLevel}
     src = tmp_path / "sizes.c"
     src.write_text('#include <stdio.h>\n#include "openludwig_b200.h"\nint main(void){\n' +
                    "".join(f'printf("%zu\\n", sizeof({n}));\n' for n in names) + "return 0;}\n")
