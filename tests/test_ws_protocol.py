@@ -5,22 +5,26 @@ The model follows the kernels' order of operations, one step at a time, and
 runs it under random interleavings of one producer warp and three consumer
 warps:
 
-* producer: publish the descriptors (neighbour row, block id) of blocks 0
-  and 1; then for each block j: publish block j+1's descriptors (j >= 1),
-  wait until every consumer has released block j - B (B stage buffers), and
-  issue block j's copies into buffer j % B (the "landed" barrier of j);
-* consumer: wait for block j to land, barrier, read block j's descriptors
-  (spread), barrier, pull, release block j, load block j+1's out-of-block
-  values (its descriptors), update block j (its descriptors again: the
-  output address).
+* producer: publish the descriptors (neighbour row, block id, ghost row) of
+  blocks 0 and 1 and signal "ready"; then for each block j: publish block
+  j+1's descriptors (j >= 1), wait until every consumer has released block
+  j - B (B stage buffers), and issue block j's copies into buffer j % B (the
+  "landed" barrier of j);
+* consumer: wait for "ready", load block 0's out-of-block values (its
+  descriptors); then for each block j: wait for it to land, write the values
+  loaded for it into its buffer (its descriptors), barrier, pull, release the
+  buffer, load block j+1's values (its descriptors), update block j (its
+  descriptors again: the output address).
 
 Checked on every step: descriptors are written only into ring slots no
-consumer still reads, and a block's copies go only into a buffer no consumer
-still pulls from; each read finds the descriptors of the block it wants.
-The ring sizes and buffer counts are read from the kernel headers.  The
-model finds the race of a double-buffered stage with a 4-slot ring: the
-producer's look-ahead then overwrites the descriptors of a block a slow
-consumer is still updating."""
+consumer still reads; a block's copies go only into a buffer that no consumer
+still writes or pulls from; a consumer writes only into a buffer no other one
+still pulls an older block from, and pulls only what every consumer has
+written; each read finds the descriptors of the block it wants.  The ring
+sizes and buffer counts are read from the kernel headers.  The model finds
+the race of a double-buffered stage with a 4-slot ring (the producer's
+look-ahead then overwrites the descriptors of a block a slow consumer is still
+updating), and those of a hand-over without the barrier or without "ready"."""
 import random
 import re
 from pathlib import Path
@@ -37,25 +41,29 @@ def _const(path: Path, name: str) -> str:
 
 
 def _params():
-    ws_ring = int(_const(CSRC / "ws.cuh", "kWsRing"))
-    tw_ring = int(_const(CSRC / "thermal_ws.cuh", "kTwRing"))
-    tw_tab = _const(CSRC / "thermal_ws.cuh", "kTwTab")
-    m = re.fullmatch(r"(\d+) \* kTwBuf", tw_tab)
-    assert m, tw_tab
-    return {"k_sc_ws": (1, ws_ring), "k_thermal_ws": (int(m.group(1)), tw_ring)}
+    out = {}
+    for kernel, header, ring, tab, buf in (
+            ("k_sc_ws", "ws.cuh", "kWsRing", "kWsTab", "kWsBuf"),
+            ("k_thermal_ws", "thermal_ws.cuh", "kTwRing", "kTwTab", "kTwBuf")):
+        m = re.fullmatch(rf"(\d+) \* {buf}", _const(CSRC / header, tab))
+        assert m, header  # the table follows the stage buffers
+        out[kernel] = (int(m.group(1)), int(_const(CSRC / header, ring)))
+    return out
 
 
 class Violation(AssertionError):
     pass
 
 
-def _run(buffers: int, ring: int, cnt: int, n_cons: int, rng: random.Random) -> None:
+def _run(buffers: int, ring: int, cnt: int, n_cons: int, rng: random.Random,
+         barrier: bool = True, wait_ready: bool = True) -> None:
     slot = [None] * ring                 # block whose descriptors a slot holds
+    ready = False                        # blocks 0 and 1 are described
     landed = [False] * cnt
     released = [0] * cnt                 # consumers that released block j
+    written = [0] * cnt                  # consumers that wrote their values of block j
     using = [set() for _ in range(n_cons)]    # blocks whose descriptors a consumer reads
-    pulling = [None] * n_cons            # block a consumer may still pull from its buffer
-    bar_count = {}                       # (barrier id, block) -> consumers arrived
+    holding = [None] * n_cons            # block whose buffer a consumer writes or pulls from
 
     def publish(p):
         for c in range(n_cons):
@@ -68,12 +76,20 @@ def _run(buffers: int, ring: int, cnt: int, n_cons: int, rng: random.Random) -> 
         if slot[p % ring] != p:
             raise Violation(f"consumer {c} reads {slot[p % ring]} instead of {p}")
 
+    def buffer_free_for(j, what):
+        for i in holding:
+            if i is not None and i != j and i % buffers == j % buffers:
+                raise Violation(f"{what} {j} overwrite buffer of {i}")
+
     def producer():
+        nonlocal ready
         publish(0)
         yield
         if cnt > 1:
             publish(1)
             yield
+        ready = True
+        yield
         for j in range(cnt):
             if 1 <= j and j + 1 < cnt:
                 publish(j + 1)
@@ -81,37 +97,40 @@ def _run(buffers: int, ring: int, cnt: int, n_cons: int, rng: random.Random) -> 
             if j >= buffers:
                 while released[j - buffers] < n_cons:
                     yield
-            for c in range(n_cons):
-                i = pulling[c]
-                if i is not None and i != j and i % buffers == j % buffers:
-                    raise Violation(f"copies of {j} overwrite buffer of {i}")
+            buffer_free_for(j, "copies of")
             landed[j] = True
             yield
 
-    def barrier(key):
-        bar_count[key] = bar_count.get(key, 0) + 1
-        while bar_count[key] < n_cons:
-            yield
+    def load(c, j):                      # out-of-block values of block j into registers
+        using[c].add(j)
+        read(c, j)
+        yield
+        read(c, j)
+        using[c].discard(j)
 
     def consumer(c):
+        while wait_ready and not ready:
+            yield
+        yield from load(c, 0)
         for j in range(cnt):
             while not landed[j]:
                 yield
-            pulling[c] = j
-            yield from barrier((1, j))
+            buffer_free_for(j, "values of")
+            holding[c] = j
             using[c].add(j)
-            read(c, j)                      # spread: neighbour row, ghost row
-            yield
-            yield from barrier((2, j))
+            read(c, j)
+            yield                           # write the values
+            written[j] += 1
+            while barrier and written[j] < n_cons:
+                yield
+            if written[j] < n_cons:
+                raise Violation(f"consumer {c} pulls block {j} before it is written")
             yield                           # pull
-            pulling[c] = None
+            holding[c] = None
             released[j] += 1
             yield
             if j + 1 < cnt:
-                using[c].add(j + 1)
-                read(c, j + 1)              # out-of-block values of block j+1
-                yield
-                using[c].discard(j + 1)
+                yield from load(c, j + 1)
             for _ in range(rng.randrange(1, 8)):   # the update, of varying length
                 read(c, j)
                 yield
@@ -135,17 +154,24 @@ def test_protocol_never_overwrites_what_a_consumer_uses(kernel):
         _run(buffers, ring, cnt=rng.randrange(1, 14), n_cons=3, rng=rng)
 
 
+def _violated(**kw) -> bool:
+    rng = random.Random(7)
+    for _ in range(400):
+        try:
+            _run(cnt=12, n_cons=3, rng=rng, **kw)
+        except Violation:
+            return True
+    return False
+
+
 @pytest.mark.parametrize("buffers,ring", [(2, 4), (1, 3)])
 def test_model_finds_the_race_of_a_short_ring(buffers, ring):
     """Too few descriptor slots for the look-ahead: two stage buffers with
     four slots, or one with three.  Some interleaving lets the producer
     overwrite a slot that a consumer still reads."""
-    rng = random.Random(7)
-    found = False
-    for _ in range(400):
-        try:
-            _run(buffers, ring, cnt=12, n_cons=3, rng=rng)
-        except Violation:
-            found = True
-            break
-    assert found
+    assert _violated(buffers=buffers, ring=ring)
+
+
+@pytest.mark.parametrize("without", ["barrier", "wait_ready"])
+def test_model_finds_a_missing_wait(without):
+    assert _violated(buffers=2, ring=8, **{without: False})
