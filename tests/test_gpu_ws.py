@@ -14,9 +14,12 @@ sum into one multiply-add in one kernel and not in the other.  So:
   largest population, 8/27) of the block kernel, and within the single-step
   oracle bar (2e-6 absolute, 1e-5 relative L2) of the oracle;
 * the two-level recursion with paired ghost rows (coarse-to-fine values),
-  4 coarse steps: relative L2 below 1e-6 on f, rho and u of both levels;
-* the block pool (batched work items, FP32 and FP16-shifted storage),
-  6 coarse steps: the same bar.
+  4 coarse steps, both operators: relative L2 below 1e-6 on f, rho and u of both
+  levels;
+* the block pool (batched work items, FP32 storage, both operators, with and
+  without WALE), 6 coarse steps: the same bar.  FP16-shifted storage has no
+  warp-specialised form: its pools keep their kernel under either choice, bit
+  for bit.
 
 Every test also checks that no bounded wait of the kernel ran out.
 """
@@ -147,11 +150,13 @@ def _recursion(hosts, p, st, steps, u, choice, max_ctas):
 
 
 @pytest.mark.parametrize("max_ctas", [0, 37], ids=["cta_per_sm", "37_ctas"])
-def test_ws_recursion_equals_block_kernel(max_ctas):
+@pytest.mark.parametrize("operator", ["cumulant", "regularized_bgk"])
+def test_ws_recursion_equals_block_kernel(operator, max_ctas):
     """Refined level inside the domain: every absent-neighbour value of the
     fine level is a ghost row written by the paired ghost pass."""
-    c, mesh, p, hosts = interior_refined_case()
+    c, mesh, p, hosts = interior_refined_case(collision_operator=operator)
     st = S.StepSettings.from_config(c, c.wall_model_enabled)
+    assert st.op == (operator == "regularized_bgk")
     a = _recursion(hosts, p, st, 4, 0.05, BLOCK, 0)
     b = _recursion(hosts, p, st, 4, 0.05, WS, max_ctas)
     for la, lb in zip(a, b):
@@ -160,17 +165,9 @@ def test_ws_recursion_equals_block_kernel(max_ctas):
             assert rel_err(y, x) < 1e-6, name
 
 
-@pytest.mark.parametrize("storage", ["f32", "f16"])
-def test_ws_block_pool_equals_block_kernel(storage):
-    """Batched work items of a two-level case and a one-level case sharing
-    the pool; the warp-specialised kernel at a grid of 11 CTAs."""
-    cases = []
-    for res, lv in ((16, 2), (8, 1)):
-        c, mesh, p, hosts = small_sphere_case(resolution=res, levels=lv,
-                                              c_wale=np.float32(0.5))
-        c.ramp_steps = 0
-        cases.append(NT.PreparedCase(c, mesh, p, hosts,
-                                     S.StepSettings.from_config(c, c.wall_model_enabled)))
+def _pool_states(cases, storage):
+    """The pool's state after 6 steps under the one-CTA-per-item kernel and
+    under the warp-specialised one at a grid of 11 CTAs."""
     out = []
     for choice, max_ctas in ((BLOCK, 0), (WS, 11)):
         _kernel(choice, max_ctas)
@@ -184,7 +181,36 @@ def test_ws_block_pool_equals_block_kernel(storage):
                 got.extend(ctx.download(cid, lvl, f=True))
         out.append(got)
         ctx.close()
-    for x, y in zip(*out):
+    return out
+
+
+def _prepared(built):
+    c, mesh, p, hosts = built
+    c.ramp_steps = 0
+    return NT.PreparedCase(c, mesh, p, hosts, S.StepSettings.from_config(c, c.wall_model_enabled))
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+def test_ws_block_pool_equals_block_kernel(storage):
+    """Batched work items of a two-level case and a one-level case sharing
+    the pool."""
+    cases = [_prepared(small_sphere_case(resolution=res, levels=lv, c_wale=np.float32(0.5)))
+             for res, lv in ((16, 2), (8, 1))]
+    for x, y in zip(*_pool_states(cases, storage)):
+        assert rel_err(y, x) < 1e-6
+        assert storage == "f32" or np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("operator,c_wale", [("regularized_bgk", 0.5), ("regularized_bgk", 0.0),
+                                             ("cumulant", 0.0)])
+def test_ws_block_pool_operators(operator, c_wale):
+    """The pool's other variants, with a refined level whose out-of-block values
+    are coarse-to-fine ghost rows beside a one-level case."""
+    kw = dict(collision_operator=operator, c_wale=np.float32(c_wale))
+    cases = [_prepared(interior_refined_case(**kw)),
+             _prepared(small_sphere_case(resolution=8, **kw))]
+    assert [c.settings.op for c in cases] == [int(operator == "regularized_bgk")] * 2
+    for x, y in zip(*_pool_states(cases, "f32")):
         assert rel_err(y, x) < 1e-6
 
 
