@@ -410,6 +410,8 @@ def pool_probe(a, local) -> None:
     from openludwig_b200 import native as NT
     from openludwig_b200 import solver as S
     storage, kernel = a.pool_probe.split(":")
+    if storage == "f16" and kernel == "ws":
+        raise SystemExit("bench.py: FP16-shifted pools have no warp-specialised kernel")
     choice = {"auto": 0, "block": 1, "ws": 2}[kernel]
     torch.cuda.set_device(local)
     cfg, mesh, p, hosts = build_case(a.workload)
@@ -491,8 +493,8 @@ def main():
     ap.add_argument("--launcher-selftest", action="store_true", help=argparse.SUPPRESS)
     ap.add_argument("--pool-probe", default=None, metavar="STORAGE:KERNEL",
                     help="time only the block pool's coarse step of the workload with storage "
-                         "f32|f16 and stream-collide kernel auto|block|ws (e.g. f16:ws), one JSON "
-                         "line")
+                         "f32|f16 and stream-collide kernel auto|block|ws (e.g. f32:ws; ws with "
+                         "f32 only), one JSON line")
     ap.add_argument("--kernel-times", action="store_true",
                     help="print the device time of each kernel per coarse step of the drop-in "
                          "path (torch profiler, warm, eager launches) instead of the bench line")
