@@ -380,8 +380,8 @@ __device__ __forceinline__ void wall_force(float dist, float rho, float ux, floa
 // update rounds alike.  kSumsPool and kSumsPoolWs (k_sc_ws) differ in one place:
 // the latter forms u_z^2 rho once, rounded, for both transforms along z.  What
 // is fused is written out (fmaf, __fmul_rn), so that no compiler's choice
-// enters.  8 steps of a pool of 6 cases: 5404 us, 5335 us with kSumsShort
-// (FP16 storage 6523 and 6438 us).
+// enters.  A pool of one cube_3lvl case, us per coarse step: 1162, with kSumsShort
+// 1148 (FP16 storage 1411 and 1386; with omega_3 = 0.9, FP32 1198 and 1191).
 // ---------------------------------------------------------------------------
 constexpr int kSumsShort = 0, kSumsPool = 1, kSumsPoolWs = 2;
 // The block pool's form (regularized BGK has one form only).
